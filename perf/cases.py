@@ -277,6 +277,32 @@ def _op(view, op, rows, cols):
     return out.conj() if op == 2 and out.is_complex() else out
 
 
+def _product(a, b):
+    """a @ b, in blocks of 16 K values summed with compensation: the rounding
+    of a long 64-bit sum would otherwise be as large as what is measured."""
+    total = torch.zeros(a.shape[0], b.shape[1], dtype=a.dtype, device=a.device)
+    lost = torch.zeros_like(total)
+    for k0 in range(0, a.shape[1], 16):
+        part = a[:, k0:k0 + 16] @ b[k0:k0 + 16] - lost
+        new = total + part
+        lost = (new - total) - part
+        total = new
+    return total
+
+
+def _solve(a, b, upper):
+    """Triangular solve by substitution, the sums in numpy's extended precision."""
+    wide = np.clongdouble if a.is_complex() else np.longdouble
+    cols = np.ascontiguousarray(a.T.cpu().numpy())  # one row per column of a
+    x = b.cpu().numpy().astype(wide)
+    n = x.size
+    for j in (range(n - 1, -1, -1) if upper else range(n)):
+        x[j] /= wide(cols[j, j])
+        rest = slice(0, j) if upper else slice(j + 1, n)
+        x[rest] -= cols[j, rest] * x[j]
+    return torch.from_numpy(x.astype(np.complex128 if a.is_complex() else np.float64)).cuda()
+
+
 def exact(case, seed):
     st = prepare(case, seed)
     kind, t = case["kind"], case["dtype"]
@@ -307,14 +333,14 @@ def exact(case, seed):
         n = case["n"]
         a = _op(up["a"].view(n, n + case["pad"]), case["trans"], n, n)
         upper = (case["uplo"] == 0) == (case["trans"] == 0)
-        return torch.linalg.solve_triangular(a, up["b"][:, None], upper=upper)[:, 0].contiguous()
+        return _solve(a, up["b"], upper)
     if kind == "gemm":
         m, n, k = case["m"], case["n"], case["k"]
         (_, ac), (_, bc), _ = _gemm_dims(case)
         a = _op(up["a"].view(ac, -1), case["op_a"], m, k)
         b = _op(up["b"].view(bc, -1), case["op_b"], k, n)
         c = up["c"].view(n, -1)[:, :m].T
-        c.copy_(ALPHA * (a @ b) + BETA * c)
+        c.copy_(ALPHA * _product(a, b) + BETA * c)
         return up["c"]
     if kind == "grouped":
         dims, ops = _batch_dims(case, 3)
