@@ -385,7 +385,7 @@ def batched_set(torch, cb, dev):
             h.set_gemm_mode(gm)
             ms = graph_time(lambda: cb.sgemm_grouped(it, count, desc))
             entry = {"ms": ms, "tflops": flops / (ms * 1e-3) / 1e12, "instances": count,
-                     "kernel": "k_gemm_simt-style FMA tiles" if gm == cb.GemmMode.NATIVE
+                     "kernel": "k_gemm_grouped (FMA tiles)" if gm == cb.GemmMode.NATIVE
                      else "k_gemm_grouped_tc (tcgen05)"}
             if gm == cb.GemmMode.SPLIT_BF16X3:
                 entry["policy_default"] = cb.grouped_config()
@@ -983,7 +983,7 @@ def run_ours(args, world, rank, local):
     if mode == cb.GemmMode.NATIVE:
         roof = {"bound": "tensor", "achieved": ach, "peak": FP32_FMA_PEAK_TFLOPS, "unit": "TFLOP/s",
                 "frac": ach / FP32_FMA_PEAK_TFLOPS, "traffic": None,
-                "kernel": "k_gemm_simt<float>", "kernel_ms": kernel_ms,
+                "kernel": "k_gemm_native<float>", "kernel_ms": kernel_ms,
                 "peak_source": "nominal FP32 FMA pipe at max clock (no measured figure)"}
     else:
         products = 3 if mode == cb.GemmMode.SPLIT_BF16X3 else 6

@@ -1,5 +1,5 @@
 // C-ABI entry points of level 3: argument checks, quick returns and the
-// dispatch between native FMA tiles and the emulated tensor-core paths
+// dispatch between the native-precision tiles and the emulated tensor-core paths
 // selected by the handle's GEMM mode.
 #include "common.cuh"
 
@@ -8,7 +8,7 @@ namespace coral {
 int gemm_bad_arg(int op_a, int op_b, size_t m, size_t n, size_t k, const void* a, size_t lda,
                  const void* b, size_t ldb, const void* c, size_t ldc, bool complex_ops);
 template <typename T>
-coral_status_t enqueue_gemm_simt(Handle* h, int op_a, int op_b, size_t m, size_t n, size_t k,
+coral_status_t enqueue_gemm_native(Handle* h, int op_a, int op_b, size_t m, size_t n, size_t k,
                                  T alpha, const T* A, size_t lda, const T* B, size_t ldb, T beta,
                                  T* C, size_t ldc);
 coral_status_t enqueue_sgemm_split(Handle* h, int terms, int op_a, int op_b, size_t m, size_t n,
@@ -49,7 +49,7 @@ coral_status_t coral_sgemm(coral_handle_t hh, int op_a, int op_b, size_t m, size
   if (compute && (H->gemm_mode == CORAL_GEMM_SPLIT_BF16X3 || H->gemm_mode == CORAL_GEMM_SPLIT_BF16X6))
     return enqueue_sgemm_split(H, H->gemm_mode == CORAL_GEMM_SPLIT_BF16X6 ? 6 : 3, op_a, op_b, m,
                                n, k, alpha, a, lda, b, ldb, beta, c, ldc);
-  return enqueue_gemm_simt<float>(H, op_a, op_b, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
+  return enqueue_gemm_native<float>(H, op_a, op_b, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
 }
 
 coral_status_t coral_dgemm(coral_handle_t hh, int op_a, int op_b, size_t m, size_t n, size_t k,
@@ -61,7 +61,7 @@ coral_status_t coral_dgemm(coral_handle_t hh, int op_a, int op_b, size_t m, size
   const bool compute = m && n && k && alpha != 0.0;
   if (compute && H->gemm_mode == CORAL_GEMM_OZAKI_INT8)
     return enqueue_dgemm_ozaki(H, op_a, op_b, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
-  return enqueue_gemm_simt<double>(H, op_a, op_b, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
+  return enqueue_gemm_native<double>(H, op_a, op_b, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
 }
 
 coral_status_t coral_cgemm(coral_handle_t hh, int op_a, int op_b, size_t m, size_t n, size_t k,
@@ -80,7 +80,7 @@ coral_status_t coral_cgemm(coral_handle_t hh, int op_a, int op_b, size_t m, size
                                n, k, al, reinterpret_cast<const float2*>(a), lda,
                                reinterpret_cast<const float2*>(b), ldb, be,
                                reinterpret_cast<float2*>(c), ldc);
-  return enqueue_gemm_simt<float2>(H, op_a, op_b, m, n, k, al, reinterpret_cast<const float2*>(a),
+  return enqueue_gemm_native<float2>(H, op_a, op_b, m, n, k, al, reinterpret_cast<const float2*>(a),
                                    lda, reinterpret_cast<const float2*>(b), ldb, be,
                                    reinterpret_cast<float2*>(c), ldc);
 }
@@ -100,7 +100,7 @@ coral_status_t coral_zgemm(coral_handle_t hh, int op_a, int op_b, size_t m, size
     return enqueue_zgemm_ozaki(H, op_a, op_b, m, n, k, al, reinterpret_cast<const double2*>(a), lda,
                                reinterpret_cast<const double2*>(b), ldb, be,
                                reinterpret_cast<double2*>(c), ldc);
-  return enqueue_gemm_simt<double2>(H, op_a, op_b, m, n, k, al, reinterpret_cast<const double2*>(a),
+  return enqueue_gemm_native<double2>(H, op_a, op_b, m, n, k, al, reinterpret_cast<const double2*>(a),
                                     lda, reinterpret_cast<const double2*>(b), ldb, be,
                                     reinterpret_cast<double2*>(c), ldc);
 }
