@@ -20,10 +20,19 @@
 // variant reads bf16 operands and accumulates in fp32.
 //
 // Batched TRSV: one CTA per instance, blocked right-looking substitution over
-// 64-row diagonal blocks: one warp solves the block (substitution, the
-// divide by the diagonal as strlsv.rs:66-140 does), then all warps subtract
-// the block's panel times the new solution from the remaining right-hand side
-// (coalesced column streaming).  Transposed operators are walked backwards.
+// 64-row diagonal blocks.  One warp runs the chain (take the previous block off
+// the next 64 rows, solve their diagonal block, divide by the diagonal as
+// strlsv.rs:66-140 does) while the other seven take that previous block off
+// all rows further down (coalesced column streaming, 48 loads in flight per
+// thread) and copy the next diagonal block and the block below it to shared
+// memory, so the chain never waits for memory.  What bounds it: the chain of
+// the largest instance (about 2.3 us per 64 rows), then HBM.  Sizes log-uniform
+// in [32, 1024], 1024 instances, 330 MB: 383 -> 106 us (3.1 TB/s); one instance
+// of 1024 rows: 387 -> 55 us.  Of that, starting the longest instances first
+// gave 40 us; asking for the next panel through L2 prefetches cost 10 us (more
+// instructions than it saved) and is not done; two rows per thread took 136 us,
+// four the same as three.  Transposed operators read the same memory by rows,
+// backward solves walk it from its end.
 #include "common.cuh"
 
 #include <cuda_bf16.h>
@@ -212,104 +221,393 @@ k_gemm_grouped(const GemmProblem* __restrict__ probs, int count, const int* __re
 // ---- batched TRSV --------------------------------------------------------------
 constexpr int kBT = 64;
 constexpr int kBTThreads = 256;
+constexpr int kBTBulk = kBTThreads - 32;   // threads of the warps beside the solving one
+constexpr int kBTLd = 68;                  // column pitch of the diagonal block (16-byte multiple)
+constexpr int kBTLs = 65;                  // and of the block below it
+constexpr int kRows = 3;                   // rows per thread of the update
+constexpr int kBTMaxX = 1024;              // right-hand sides up to here stay in shared memory
 
-__global__ void __launch_bounds__(kBTThreads, 4)
-k_trsv_batched(const TrsvProblem* __restrict__ probs, int count) {
-  __shared__ float D[kBT][kBT + 1];  // D[r][c] = op(A)(b0 + r, b0 + c)
-  __shared__ float xb[kBT];
-  const int pi = blockIdx.x;
-  if (pi >= count) return;
+struct TrsvSmem {
+  float D[2][kBT][kBTLd];   // [column][row]
+  float S[2][kBT][kBTLs];   // [column][row]
+  float xb[2][kBT];
+  float part[4][kBT];
+  float inv[kBT];
+  float x[kBTMaxX];
+};
+
+// The system in solve order: always lower triangular, element (i, j) of op(A)
+// at a[i * rs + j * cs], right-hand side i at x[i * xs].  A backward solve
+// walks the same memory from its end.
+struct TrsvView {
+  const float* a;
+  float* x;
+  long long rs, cs, xs;
+  int n;
+};
+
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// Starts the copy of diagonal block b (lower half) and of the block below the
+// previous diagonal (rows of block b, columns of block b - 1); warp w of
+// `warps`, lanes along the stored direction.
+__device__ __forceinline__ void trsv_fetch(const TrsvView& v, int b, bool below, TrsvSmem& sm, int w, int warps,
+                                           bool rows_first) {
+  const int b0 = b * kBT, bn = min(kBT, v.n - b0), lane = threadIdx.x & 31;
+  const float* diag = v.a + b0 * (v.rs + v.cs);
+  const float* left = diag - kBT * v.cs;
+  float(*D)[kBTLd] = sm.D[b & 1];
+  float(*S)[kBTLs] = sm.S[(b - 1) & 1];
+  if (rows_first) {
+    const bool in0 = lane < bn, in1 = lane + 32 < bn;
+    diag += lane * v.rs;
+    left += lane * v.rs;
+    for (int c = w; c < kBT; c += warps) {
+      const long long o = c * v.cs;
+      if (in0 && c <= lane) cp_async4(&D[c][lane], diag + o);
+      if (in1 && c <= lane + 32) cp_async4(&D[c][lane + 32], diag + o + 32 * v.rs);
+      if (below) {
+        if (in0) cp_async4(&S[c][lane], left + o);
+        if (in1) cp_async4(&S[c][lane + 32], left + o + 32 * v.rs);
+      }
+    }
+  } else {
+    diag += lane * v.cs;
+    left += lane * v.cs;
+    for (int r = w; r < bn; r += warps) {
+      const long long o = r * v.rs;
+      if (lane <= r) cp_async4(&D[lane][r], diag + o);
+      if (lane + 32 <= r) cp_async4(&D[lane + 32][r], diag + o + 32 * v.cs);
+      if (below) {
+        cp_async4(&S[lane][r], left + o);
+        cp_async4(&S[lane + 32][r], left + o + 32 * v.cs);
+      }
+    }
+  }
+}
+
+// Zeros what the copies of a last, short block b leave untouched: rows past the
+// system then solve to 0 and take nothing from the others.
+__device__ __forceinline__ void trsv_pad(TrsvSmem& sm, int b, int bn) {
+  float(*D)[kBTLd] = sm.D[b & 1];
+  float(*S)[kBTLs] = sm.S[(b - 1) & 1];
+  for (int e = threadIdx.x; e < kBT * kBT; e += kBTThreads) {
+    const int r = e % kBT, c = e / kBT;
+    if (r >= bn) {
+      if (c <= r) D[c][r] = r == c ? 1.f : 0.f;
+      S[c][r] = 0.f;
+    }
+  }
+}
+
+// Reciprocal of the diagonal entry of row r (one thread per row), 1 for a unit
+// diagonal; returns whether the product with it can stand for the division.
+__device__ __forceinline__ bool trsv_recip(TrsvSmem& sm, int b, int r, bool unit) {
+  float(*D)[kBTLd] = sm.D[b & 1];
+  if (unit) D[r][r] = 1.f;
+  const float d = unit ? 1.f : D[r][r];
+  sm.inv[r] = 1.f / d;
+  return fabsf(d) > 0x1p-60f && fabsf(d) < 0x1p60f;
+}
+
+// One warp: solves diagonal block b for the right-hand sides rh[h] of rows
+// lane + 32 h, 8 rows at a time.  Every lane solves the 8 x 8 corner (no
+// exchange inside its chain), then takes its 8 products off its own rows.
+// x / d is x * (1 / d) with one residual correction.  Where that could round
+// differently -- a diagonal far from 1 (!fast), or a result that is not finite,
+// which reaches every later row -- the block is solved again with divisions.
+__device__ __forceinline__ void trsv_solve(TrsvSmem& sm, int b, bool fast, const float (&rhs)[2]) {
+  const int lane = threadIdx.x & 31;
+  const float(*D)[kBTLd] = sm.D[b & 1];
+  float rh[2] = {rhs[0], rhs[1]}, last = 0.f;
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    float q[8], xs[8], l[8][8], iv[8], o[2][8];  // corner: right-hand sides, solution; own rows
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (j < 4) *reinterpret_cast<float4*>(l[j]) = *reinterpret_cast<const float4*>(&D[8 * s + j][8 * s]);
+      *reinterpret_cast<float4*>(l[j] + 4) = *reinterpret_cast<const float4*>(&D[8 * s + j][8 * s + 4]);
+    }
+    *reinterpret_cast<float4*>(iv) = *reinterpret_cast<const float4*>(&sm.inv[8 * s]);
+    *reinterpret_cast<float4*>(iv + 4) = *reinterpret_cast<const float4*>(&sm.inv[8 * s + 4]);
+#pragma unroll
+    for (int h = s / 4; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[h][j] = D[8 * s + j][lane + 32 * h];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q[j] = __shfl_sync(0xffffffffu, rh[s / 4], (8 * s + j) & 31);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float t = q[j] * iv[j];
+      xs[j] = fmaf(fmaf(-t, l[j][j], q[j]), iv[j], t);
+#pragma unroll
+      for (int i = j + 1; i < 8; ++i) q[i] = fmaf(-l[j][i], xs[j], q[i]);
+    }
+    last = xs[7];
+    float mine = xs[0];
+#pragma unroll
+    for (int j = 1; j < 8; ++j) mine = (lane & 7) == j ? xs[j] : mine;
+#pragma unroll
+    for (int h = s / 4; h < 2; ++h) {
+      float a = rh[h], c = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        a = fmaf(-o[h][j], xs[j], a);
+        c = fmaf(-o[h][4 + j], xs[4 + j], c);
+      }
+      if (lane + 32 * h >= 8 * s + 8) rh[h] = a + c;
+    }
+    if ((lane >> 3) == (s & 3)) rh[s / 4] = mine;
+  }
+  if (!(fast && fabsf(last) < INFINITY)) {
+    rh[0] = rhs[0];
+    rh[1] = rhs[1];
+#pragma unroll 1
+    for (int j = 0; j < kBT; ++j) {
+      const float x = __shfl_sync(0xffffffffu, j < 32 ? rh[0] : rh[1], j & 31) / D[j][j];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = lane + 32 * h;
+        if (r == j) rh[h] = x;
+        if (r > j) rh[h] = fmaf(-D[j][r], x, rh[h]);
+      }
+    }
+  }
+  float* xb = sm.xb[b & 1];
+  xb[lane] = rh[0];
+  xb[lane + 32] = rh[1];
+  __syncwarp();
+}
+
+// Instance for a CTA: within each window of kBTWindow instances, the CTAs take
+// them in decreasing order of size class (quarters of an octave, input order
+// inside a class), so the longest solves start first.  Every CTA finds its own
+// instance from the window's sizes: no plan pass, no memory beyond its own.
+constexpr int kBTWindow = 1024, kBTClasses = 128;
+__device__ __forceinline__ int trsv_class(int n) {
+  if (n <= 0) return 0;
+  const int lg = 31 - __clz(n);
+  return lg * 4 + (lg >= 2 ? (n >> (lg - 2)) & 3 : 0);
+}
+__device__ __forceinline__ int trsv_pick(const TrsvProblem* __restrict__ probs, int count, int pos) {
+  constexpr int kPer = kBTWindow / kBTThreads;
+  __shared__ int hist[kBTClasses], warp_sum[kBTThreads / 32];
+  __shared__ int cls, rank, pick;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int base = pos / kBTWindow * kBTWindow, local = pos - base;
+  if (t < kBTClasses) hist[t] = 0;
+  int key[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int i = base + t * kPer + q;
+    key[q] = i < count ? trsv_class(probs[i].n) : -1;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kPer; ++q)
+    if (key[q] >= 0) atomicAdd(&hist[key[q]], 1);
+  __syncthreads();
+  if (warp == 0) {  // classes from the top, 4 per lane
+    int h[4], sum = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sum += h[q] = hist[kBTClasses - 1 - (lane * 4 + q)];
+    int before = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += u;
+    }
+    before -= sum;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (local >= before && local < before + h[q]) {
+        cls = kBTClasses - 1 - (lane * 4 + q);
+        rank = local - before;
+      }
+      before += h[q];
+    }
+  }
+  __syncthreads();
+  int mine = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) mine += key[q] == cls;
+  int before = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += u;
+  }
+  if (lane == 31) warp_sum[warp] = before;
+  __syncthreads();
+  before -= mine;
+  for (int w = 0; w < warp; ++w) before += warp_sum[w];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q)
+    if (key[q] == cls && before++ == rank) pick = base + t * kPer + q;
+  __syncthreads();
+  return pick;
+}
+
+__global__ void __launch_bounds__(kBTThreads, 2)
+k_trsv_batched(const TrsvProblem* __restrict__ probs, int count, bool ordered) {
+  extern __shared__ __align__(16) unsigned char trsv_smem[];
+  TrsvSmem& sm = *reinterpret_cast<TrsvSmem*>(trsv_smem);
+  if ((int)blockIdx.x >= count) return;
+  const int pi = ordered ? trsv_pick(probs, count, blockIdx.x) : (int)blockIdx.x;
   const TrsvProblem p = probs[pi];
-  const int n = p.n;
-  if (n <= 0) return;
+  if (p.n <= 0) return;
   const bool t = p.trans != CORAL_NO_TRANSPOSE;
   const bool lower_eff = (p.uplo == CORAL_LOWER) != t;
   const bool unit = p.diag == CORAL_UNIT;
-  const float* A = p.a;
-  float* x = p.x;
-  const size_t lda = p.lda, incx = p.incx;
-  auto opA = [&](int r, int c) -> float {  // op(A)(r, c)
-    return t ? A[c + (size_t)r * lda] : A[r + (size_t)c * lda];
-  };
-  const int nblk = (n + kBT - 1) / kBT;
-  for (int bi = 0; bi < nblk; ++bi) {
-    const int blk = lower_eff ? bi : nblk - 1 - bi;
-    const int b0 = blk * kBT, bn = min(kBT, n - b0);
-    // stage the diagonal block of op(A): loads in groups of 8 before their
-    // stores, so the block costs two memory round trips
+  TrsvView v;
+  v.n = p.n;
+  v.rs = t ? p.lda : 1;
+  v.cs = t ? 1 : p.lda;
+  v.xs = p.incx;
+  v.a = p.a;
+  v.x = p.x;
+  if (!lower_eff) {
+    v.a += (long long)(p.n - 1) * (1 + p.lda);
+    v.x += (long long)(p.n - 1) * p.incx;
+    v.rs = -v.rs;
+    v.cs = -v.cs;
+    v.xs = -v.xs;
+  }
+  const int n = v.n, nblk = (n + kBT - 1) / kBT;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool in_smem = n <= kBTMaxX;
+
+  trsv_fetch(v, 0, false, sm, warp, kBTThreads / 32, !t);
+  if (nblk > 1) trsv_fetch(v, 1, true, sm, warp, kBTThreads / 32, !t);
+  if (in_smem)
+    for (int i = threadIdx.x; i < n; i += kBTThreads) sm.x[i] = v.x[i * v.xs];
+  auto rhs = [&](int i) { return i >= n ? 0.f : in_smem ? sm.x[i] : v.x[i * v.xs]; };
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (n < kBT) trsv_pad(sm, 0, n);
+  else if (nblk == 2 && n < 2 * kBT) trsv_pad(sm, 1, n - kBT);
+  __syncthreads();
+  bool ok = true;
+  if (threadIdx.x < kBT) ok = trsv_recip(sm, 0, threadIdx.x, unit);
+  bool fast = __syncthreads_and(ok);
+  if (warp == 0) {
+    const float r2[2] = {rhs(lane), rhs(lane + 32)};
+    trsv_solve(sm, 0, fast, r2);
+    if (lane < n) v.x[lane * v.xs] = sm.xb[0][lane];
+    if (lane + 32 < n) v.x[(lane + 32) * v.xs] = sm.xb[0][lane + 32];
+  }
+  __syncthreads();
+  for (int b = 0; b + 1 < nblk; ++b) {
+    const float* xb = sm.xb[b & 1];
+    // Rows of block b + 1: everything up to block b - 1 is already off them;
+    // take block b off (4 threads a row, every warp), then one warp solves.
+    const int b1 = (b + 1) * kBT;
+    {
+      const float(*S)[kBTLs] = sm.S[b & 1];
+      const int row = threadIdx.x % kBT, part = threadIdx.x / kBT;  // a warp: 32 rows, 16 columns
+      float a0 = 0.f, a1 = 0.f;
 #pragma unroll
-    for (int q0 = 0; q0 < kBT * kBT / kBTThreads; q0 += 8) {
-      float dv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int e = threadIdx.x + (q0 + q) * kBTThreads;
-        const int r = e % kBT, c = e / kBT;
-        dv[q] = (r < bn && c < bn) ? (t ? A[(b0 + c) + (size_t)(b0 + r) * lda] : A[(b0 + r) + (size_t)(b0 + c) * lda])
-                                   : 0.f;
+      for (int c = 0; c < 16; c += 4) {
+        const float4 x4 = *reinterpret_cast<const float4*>(xb + part * 16 + c);
+        a0 = fmaf(S[part * 16 + c][row], x4.x, a0);
+        a1 = fmaf(S[part * 16 + c + 1][row], x4.y, a1);
+        a0 = fmaf(S[part * 16 + c + 2][row], x4.z, a0);
+        a1 = fmaf(S[part * 16 + c + 3][row], x4.w, a1);
       }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int e = threadIdx.x + (q0 + q) * kBTThreads;
-        D[e % kBT][e / kBT] = dv[q];
-      }
+      sm.part[part][row] = a0 + a1;
+      ok = part != 3 || trsv_recip(sm, b + 1, row, unit);
     }
-    if (threadIdx.x < kBT) xb[threadIdx.x] = threadIdx.x < bn ? x[(size_t)(b0 + threadIdx.x) * incx] : 0.f;
-    __syncthreads();
-    // warp 0: substitution on the diagonal block (lane owns rows lane, lane+32)
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
-      float r0 = xb[lane], r1 = xb[lane + 32];
-      for (int s = 0; s < bn; ++s) {
-        const int j = lower_eff ? s : bn - 1 - s;
-        const int owner = j & 31;
-        float xj = (j < 32) ? r0 : r1;
-        xj = __shfl_sync(0xffffffffu, xj, owner);
-        if (!unit) xj = xj / D[j][j];
-        if (lane == owner) {
-          if (j < 32) r0 = xj; else r1 = xj;
-        }
-        // eliminate column j from the rows still to be solved
-        const int i0 = lane, i1 = lane + 32;
-        if (lower_eff) {
-          if (i0 > j && i0 < bn) r0 = fmaf(-D[i0][j], xj, r0);
-          if (i1 > j && i1 < bn) r1 = fmaf(-D[i1][j], xj, r1);
-        } else {
-          if (i0 < j) r0 = fmaf(-D[i0][j], xj, r0);
-          if (i1 < j) r1 = fmaf(-D[i1][j], xj, r1);
-        }
+    fast = __syncthreads_and(ok);
+    if (warp == 0) {
+      float r2[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = lane + 32 * h;
+        r2[h] = rhs(b1 + r) - ((sm.part[0][r] + sm.part[1][r]) + (sm.part[2][r] + sm.part[3][r]));
       }
-      xb[lane] = r0;
-      xb[lane + 32] = r1;
-    }
-    __syncthreads();
-    if (threadIdx.x < bn) x[(size_t)(b0 + threadIdx.x) * incx] = xb[threadIdx.x];
-    // update the rows still to be solved: rhs_i -= sum_c op(A)(i, b0 + c) xb[c]
-    const int r_lo = lower_eff ? b0 + bn : 0, r_hi = lower_eff ? n : b0;
-    // Two rows at a time, their loads 16 per row before the sums (a single
-    // CTA solves the largest instances, so its memory parallelism sets the
-    // batch's tail)
-    for (int i = r_lo + threadIdx.x; i < r_hi; i += 2 * kBTThreads) {
-      const int i2 = i + kBTThreads;
-      const bool two = i2 < r_hi;
-      float s4[4] = {0.f, 0.f, 0.f, 0.f}, u4[4] = {0.f, 0.f, 0.f, 0.f};
+      trsv_solve(sm, b + 1, fast, r2);
+      const float* xn = sm.xb[(b + 1) & 1];
+      if (b1 + lane < n) v.x[(b1 + lane) * v.xs] = xn[lane];
+      if (b1 + lane + 32 < n) v.x[(b1 + lane + 32) * v.xs] = xn[lane + 32];
+    } else {
+      const int tb = threadIdx.x - 32;
+      if (b + 2 < nblk) trsv_fetch(v, b + 2, true, sm, warp - 1, kBTBulk / 32, !t);
+      const int lo = (b + 2) * kBT;
+      const float* col = v.a + (long long)b * kBT * v.cs;
+      if (!t) {
+        // kRows rows per thread, 16 loads per row before their sums
+        for (int i = lo + tb; i < n; i += kRows * kBTBulk) {
+          const float* pr[kRows];
+#pragma unroll
+          for (int q = 0; q < kRows; ++q) pr[q] = col + min(i + q * kBTBulk, n - 1) * v.rs;
+          const int rows = min(kRows, (n - i + kBTBulk - 1) / kBTBulk);
+          float sum[kRows][2] = {};
 #pragma unroll 1
-      for (int c0 = 0; c0 < kBT; c0 += 16) {
-        float a[16], b[16];
+          for (int c0 = 0; c0 < kBT; c0 += 16) {
+            float a[kRows][16];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          a[c] = c0 + c < bn ? opA(i, b0 + c0 + c) : 0.f;
-          b[c] = two && c0 + c < bn ? opA(i2, b0 + c0 + c) : 0.f;
+            for (int q = 0; q < kRows; ++q)
+              if (q < rows)
+#pragma unroll
+                for (int c = 0; c < 16; ++c) a[q][c] = pr[q][(c0 + c) * v.cs];
+#pragma unroll
+            for (int c = 0; c < 16; c += 4) {
+              const float4 x4 = *reinterpret_cast<const float4*>(xb + c0 + c);
+#pragma unroll
+              for (int q = 0; q < kRows; ++q)
+                if (q < rows) {
+                  sum[q][0] = fmaf(a[q][c], x4.x, sum[q][0]);
+                  sum[q][1] = fmaf(a[q][c + 1], x4.y, sum[q][1]);
+                  sum[q][0] = fmaf(a[q][c + 2], x4.z, sum[q][0]);
+                  sum[q][1] = fmaf(a[q][c + 3], x4.w, sum[q][1]);
+                }
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < kRows; ++q)
+            if (q < rows) {
+              const int k = i + q * kBTBulk;
+              if (in_smem) sm.x[k] -= sum[q][0] + sum[q][1];
+              else v.x[k * v.xs] -= sum[q][0] + sum[q][1];
+            }
         }
+      } else {
+        // stored along the row: a warp reads 8 rows, lanes along the columns
+        const float x0 = xb[lane], x1 = xb[lane + 32];
+        for (int i = lo + (warp - 1) * 8; i < n; i += (kBTBulk / 32) * 8) {
+          float a[8], d[8];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          s4[c & 3] = fmaf(a[c], xb[c0 + c], s4[c & 3]);
-          u4[c & 3] = fmaf(b[c], xb[c0 + c], u4[c & 3]);
+          for (int r = 0; r < 8; ++r) {
+            const float* pr = col + min(i + r, n - 1) * v.rs;
+            a[r] = pr[lane * v.cs];
+            d[r] = pr[(lane + 32) * v.cs];
+          }
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            float sum = fmaf(d[r], x1, a[r] * x0);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            a[r] = sum;
+          }
+          float mine = a[0];
+#pragma unroll
+          for (int r = 1; r < 8; ++r) mine = lane == r ? a[r] : mine;
+          if (lane < 8 && i + lane < n) {
+            if (in_smem) sm.x[i + lane] -= mine;
+            else v.x[(i + lane) * v.xs] -= mine;
+          }
         }
       }
-      x[(size_t)i * incx] -= (s4[0] + s4[1]) + (s4[2] + s4[3]);
-      if (two) x[(size_t)i2 * incx] -= (u4[0] + u4[1]) + (u4[2] + u4[3]);
+      asm volatile("cp.async.wait_all;" ::: "memory");
     }
+    // (the last block's copies were waited for by the threads that made them)
     __syncthreads();
+    if (b + 3 == nblk && n < nblk * kBT) {
+      trsv_pad(sm, nblk - 1, n - (nblk - 1) * kBT);
+      __syncthreads();
+    }
   }
 }
 
@@ -374,9 +672,16 @@ coral_status_t coral_strsv_batched(coral_handle_t hh, size_t count,
   if (count == 0) return CORAL_OK;
   if (!problems) return bad_arg(H, 2);
   if (count > (size_t)INT32_MAX) return CORAL_ERR_NOT_SUPPORTED;
+  static uint64_t attr_devices = 0;  // bit d: attribute set on device d
+  const uint64_t bit = H->device < 64 ? (1ull << H->device) : 0;
+  if (!(attr_devices & bit) || !bit) {
+    CORAL_CUDA(H, cudaFuncSetAttribute(k_trsv_batched, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(TrsvSmem)));
+    attr_devices |= bit;
+  }
   timed_begin(H);
-  k_trsv_batched<<<(unsigned)count, kBTThreads, 0, H->stream>>>(
-      reinterpret_cast<const TrsvProblem*>(problems), (int)count);
+  k_trsv_batched<<<(unsigned)count, kBTThreads, sizeof(TrsvSmem), H->stream>>>(
+      reinterpret_cast<const TrsvProblem*>(problems), (int)count, count > (size_t)H->sm_count * 2);
   coral_status_t s = launch_status(H);
   timed_end(H);
   return s;
