@@ -10,15 +10,11 @@
 //
 // The instances' operands have arbitrary leading dimensions and alignments,
 // which tensor maps cannot describe without per-instance host work, so the
-// operands are staged by producer warps instead of TMA: each thread takes
-// items of 8 consecutive K values of one row -- one contiguous segment (16-byte
-// loads where it is aligned) for an operand stored along K, or 8 row-coalesced
-// loads for one stored along the rows -- converts them to bf16 pieces in
-// registers, and writes each piece with one 16-byte shared store into the
-// K-major 64-byte-swizzled layout that a TMA
-// CU_TENSOR_MAP_SWIZZLE_64B load would write (rows of 32 bf16, 8-row / 512-byte
-// atoms, 16-byte chunk c of row r at chunk c ^ ((r >> 1) & 3)), so the MMA
-// descriptors are the same as the TMA-fed kernels'.
+// operands are staged by producer warps instead of TMA: blocks of 32 rows x 32
+// K values, read in runs of consecutive elements whichever way the operand is
+// stored, converted to bf16 pieces in registers and written into the K-major
+// 64-byte-swizzled layout that a TMA CU_TENSOR_MAP_SWIZZLE_64B load would write,
+// so the MMA descriptors are the same as the TMA-fed kernels'.
 //
 // Plan (k_grouped_plan, one CTA): every instance gets a tile width BN from the
 // handle's per-class policy (classes by n: <= 64, <= 128, <= 256, > 256;
@@ -26,21 +22,30 @@
 // overrides it), instances are ordered by decreasing K bucket (longest tiles
 // first), and the exclusive prefix sum of 128 x BN output tiles is formed.
 //
-// GEMM (k_gemm_grouped_tc, persistent, one CTA per SM, 22 warps):
-//   warp 0      scheduler: takes tile indices from a global atomic counter
-//               (dynamic load balance), decodes (instance, m0, n0, BN) and
-//               publishes them through a 16-deep shared queue;
-//   warps 1-16  producers: stage the K slabs of each tile into a ring of
-//               shared-memory stages (4 for fp32 pieces, 8 for bf16), each
-//               thread issuing all its loads of a slab before converting any;
+// GEMM (k_gemm_grouped_tc, persistent, one CTA per SM, 26 warps):
+//   warp 0      scheduler: takes up to 4 tile indices at once from a global
+//               atomic counter (dynamic load balance), finds their instances
+//               with 8 lanes each, and publishes tile and descriptor through
+//               a 16-deep shared queue (one tile at a time by one lane took
+//               5 us a tile and bound the kernel at 310 us);
+//   warps 1-16  producers, four groups: A of even slabs, A of odd ones, B of
+//               even, B of odd, into a ring of shared-memory stages (4 for fp32
+//               pieces, 8 for bf16); they also ask for the tile's C in L2;
 //   warp 17     MMA issuer (lane 0): tcgen05.mma M=128, N=BN, K=16 into one of
 //               two TMEM accumulators of 256 columns, in chunks of at most
 //               32 slabs (1024 K) per accumulation;
-//   warps 18-21 epilogue: tcgen05.ld the accumulator (thread = row), apply
-//               alpha / beta to C with coalesced column accesses (the C loads
-//               of 16 columns issued together before their stores, so a tile
-//               costs a few memory round trips, not one per column); chunks
-//               after the first add alpha * partial into C.
+//   warps 18-25 epilogue: tcgen05.ld the accumulator (thread = row, the two
+//               warps of a quadrant on alternate 16 columns), apply alpha / beta
+//               to C with coalesced column accesses, the C loads of the next 16
+//               columns ahead of this group's stores; chunks after the first
+//               add alpha * partial into C.
+// Bound: issue slots (55% busy, a quarter of the stalls on instruction fetch)
+// and the latency of the slabs; 4096 instances with sizes log-uniform in
+// [16, 512] (1.34 GB, a floor of 208 us): fp32 810 -> 488 us, bf16 807 -> 436.
+// 2000 of 128^3: 197 -> 111 us.  Timed apart (the other side's work left out):
+// producers 350 us, epilogue 295, control alone 190.  A batch of four
+// instances of 2000-2300 is 10% slower than with the earlier 16-byte loads
+// (570 -> 631 us): such sizes belong to coral_sgemm.
 // Every wait is bounded: a wait that gives up sets the handle's status word
 // (reported by coral_sync) and the CTA winds down.
 #include "common.cuh"
@@ -57,11 +62,12 @@ constexpr int kTM = 128;          // tile rows (TMEM lanes)
 constexpr int kTK = 32;           // K slab: one 64-byte swizzled row of bf16
 constexpr int kMaxBN = 256;
 constexpr int kProdWarps = 16;
-constexpr int kEpiWarps = 4;
+constexpr int kEpiWarps = 8;
 constexpr int kMmaWarp = 1 + kProdWarps;
 constexpr int kEpiWarp0 = kMmaWarp + 1;
-constexpr int kTcThreads = 32 * (kEpiWarp0 + kEpiWarps);  // 704
+constexpr int kTcThreads = 32 * (kEpiWarp0 + kEpiWarps);  // 832
 constexpr int kQueue = 16;
+constexpr int kBatch = 4;   // tiles the scheduler looks up at once
 constexpr int kChunkSlabs = 32;
 constexpr uint32_t kAPieceBytes = kTM * kTK * 2;       // 8 KiB
 constexpr uint32_t kBPieceBytes = kMaxBN * kTK * 2;    // 16 KiB
@@ -90,9 +96,10 @@ template <int NPC>
 constexpr size_t tc_smem_bytes() { return (size_t)TcCfg<NPC>::kStages * tc_stage_bytes<NPC>() + 1024; }
 
 struct TileInfo {
-  int inst;    // instance, -1: no more tiles
+  int more;    // 0: no more tiles
   int m0, n0, bn;
   int nslabs;  // K slabs; 0: scale-only tile (alpha == 0 or k == 0)
+  coral_sgemm_problem_t p;  // the instance
 };
 
 __device__ __forceinline__ int policy_bn(const GroupedPolicy& pol, const coral_sgemm_problem_t& p) {
@@ -103,263 +110,237 @@ __device__ __forceinline__ int policy_bn(const GroupedPolicy& pol, const coral_s
 
 // One CTA.  order[pos] = instance, bn_pos[pos] = its tile width, prefix[pos] =
 // tiles before position pos (prefix[count] = total).  Positions follow
-// decreasing K bucket, so the longest tiles are handed out first.
-__global__ void __launch_bounds__(1024)
+// decreasing K bucket, so the longest tiles are handed out first.  K falls in a
+// few buckets, so the shared counters are taken once per bucket and warp, not
+// once per lane, and the prefix sum is one scan over per-thread runs (4096
+// instances: 18 us with a counter access per lane and a scan per 1024).
+__global__ void __launch_bounds__(1024, 1)
 k_grouped_plan(const coral_sgemm_problem_t* __restrict__ probs, int count, GroupedPolicy pol,
                int* __restrict__ order, int* __restrict__ bn_pos, long long* __restrict__ prefix) {
-  __shared__ int hist[32], start[32], cursor[32];
+  __shared__ int hist[32], cursor[32];
   __shared__ long long warp_tot[32];
-  __shared__ long long carry;
-  if (threadIdx.x < 32) { hist[threadIdx.x] = 0; cursor[threadIdx.x] = 0; }
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  auto key_of = [&](const coral_sgemm_problem_t& p) {
-    if (p.m <= 0 || p.n <= 0 || p.k <= 0 || p.alpha == 0.f) return 0;
-    return 31 - __clz(p.k);
-  };
-  for (int i = threadIdx.x; i < count; i += blockDim.x) atomicAdd(&hist[key_of(probs[i])], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int b = 31; b >= 0; --b) { start[b] = s; s += hist[b]; }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < count; i += blockDim.x) {
-    const int b = key_of(probs[i]);
-    order[start[b] + atomicAdd(&cursor[b], 1)] = i;
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int base = 0; base < count; base += blockDim.x) {
-    const int pos = base + threadIdx.x;
-    long long t = 0;
-    if (pos < count) {
-      const coral_sgemm_problem_t p = probs[order[pos]];
-      const int bn = policy_bn(pol, p);
-      bn_pos[pos] = bn;
-      if (p.m > 0 && p.n > 0) t = (long long)((p.m + kTM - 1) / kTM) * ((p.n + bn - 1) / bn);
+  if (threadIdx.x < 32) hist[threadIdx.x] = 0;
+  __syncthreads();
+  // what the plan needs of instance i, in two 16-byte loads where they are aligned
+  struct Entry { int key, bn; long long tiles; };
+  const bool vec = (reinterpret_cast<uintptr_t>(probs) & 15) == 0;
+  auto fetch = [&](int i) -> Entry {
+    if (i >= count) return {-1, 0, 0};
+    coral_sgemm_problem_t p;
+    int4 w[2];
+    const int4* src = reinterpret_cast<const int4*>(probs + i);
+    if (vec) {
+      w[0] = src[0];
+      w[1] = src[1];
+    } else {
+      const int2* s2 = reinterpret_cast<const int2*>(src);
+      const int2 a = s2[0], b = s2[1], c = s2[2], d = s2[3];
+      w[0] = make_int4(a.x, a.y, b.x, b.y);
+      w[1] = make_int4(c.x, c.y, d.x, d.y);
     }
-    long long v = t;
+    p.m = w[0].z;
+    p.n = w[0].w;
+    p.k = w[1].x;
+    p.alpha = __int_as_float(w[1].y);
+    p.reserved = w[1].w;
+    Entry e;
+    e.key = p.m <= 0 || p.n <= 0 || p.k <= 0 || p.alpha == 0.f ? 0 : 31 - __clz(p.k);
+    e.bn = policy_bn(pol, p);
+    e.tiles = p.m > 0 && p.n > 0 ? (((long long)p.m + kTM - 1) / kTM) * (((long long)p.n + e.bn - 1) / e.bn) : 0;
+    return e;
+  };
+  auto count_key = [&](int key) {
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    if (key >= 0 && lane == __ffs(peers) - 1) atomicAdd(&hist[key], __popc(peers));
+  };
+  auto place = [&](int i, const Entry& e) {
+    const unsigned peers = __match_any_sync(0xffffffffu, e.key);
+    const int leader = __ffs(peers) - 1;
+    int pos = 0;
+    if (e.key >= 0 && lane == leader) pos = atomicAdd(&cursor[e.key], __popc(peers));
+    pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(peers & ((1u << lane) - 1u));
+    if (e.key >= 0) {
+      order[pos] = i;
+      bn_pos[pos] = e.bn;
+      prefix[pos] = e.tiles;  // replaced by the sum below
+    }
+  };
+  // up to 4096 instances stay in registers between the two passes
+  constexpr int kKept = 4;
+  const int rounds = (count + 1023) / 1024;
+  Entry kept[kKept];
+#pragma unroll
+  for (int q = 0; q < kKept; ++q) kept[q] = fetch(q * 1024 + threadIdx.x);
+#pragma unroll
+  for (int q = 0; q < kKept; ++q)
+    if (q < rounds) count_key(kept[q].key);
+  for (int q = kKept; q < rounds; ++q) count_key(fetch(q * 1024 + threadIdx.x).key);
+  __syncthreads();
+  if (w == 0) {  // first position of each bucket, the deepest first
+    int before = hist[31 - lane];
+    const int own = before;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const long long u = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += u;
+      const int u = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += u;
     }
-    if (lane == 31) warp_tot[w] = v;
-    __syncthreads();
-    if (w == 0) {
-      long long s = lane < (int)(blockDim.x >> 5) ? warp_tot[lane] : 0;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const long long u = __shfl_up_sync(0xffffffffu, s, o);
-        if (lane >= o) s += u;
-      }
-      warp_tot[lane] = s;
-    }
-    __syncthreads();
-    const long long excl = carry + (w ? warp_tot[w - 1] : 0) + v - t;
-    if (pos < count) prefix[pos] = excl;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = excl + t;
-    __syncthreads();
+    cursor[31 - lane] = before - own;
   }
-  if (threadIdx.x == 0) prefix[count] = carry;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kKept; ++q)
+    if (q < rounds) place(q * 1024 + threadIdx.x, kept[q]);
+  for (int q = kKept; q < rounds; ++q) place(q * 1024 + threadIdx.x, fetch(q * 1024 + threadIdx.x));
+  __syncthreads();
+  const int per = (count + 1023) / 1024, lo = threadIdx.x * per, hi = min(count, lo + per);
+  long long own = 0;
+  for (int pos = lo; pos < hi; ++pos) own += prefix[pos];
+  long long v = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  if (lane == 31) warp_tot[w] = v;
+  __syncthreads();
+  if (w == 0) {
+    long long t = warp_tot[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += u;
+    }
+    warp_tot[lane] = t;
+  }
+  __syncthreads();
+  long long run = (w ? warp_tot[w - 1] : 0) + v - own;
+  for (int pos = lo; pos < hi; ++pos) {
+    const long long t = prefix[pos];
+    prefix[pos] = run;
+    run += t;
+  }
+  if (threadIdx.x == 1023) prefix[count] = run;
 }
 
-template <typename TIn> __device__ __forceinline__ float ld_val(const TIn* p);
-template <> __device__ __forceinline__ float ld_val<float>(const float* p) { return __ldg(p); }
+// ---- producers' staging -------------------------------------------------------
+// A group of 4 warps stages one operand of every other slab, 32 rows at a time
+// (a "block"): each thread takes 8 values of a block, and the loads of
+// kInFlight blocks are issued before any value is converted.  How the 8 values
+// lie follows the operand's storage, so that every warp load reads one or two
+// runs of consecutive elements:
+//   along the rows:  one row (lane), 8 consecutive K values (one chunk per warp);
+//   along K:         4 rows (2 apart), 2 consecutive K values (16 lanes a row).
+// Either way value j lies (j >> 1) * s1 + (j & 1) * s0 from the first, so one
+// piece of code loads both, and everything else is fixed per tile or moves by
+// a fixed step from slab to slab: with the kernel bound by issue slots, not by
+// memory, what a block costs is the instructions around its 8 loads.
+constexpr int kGroups = 4, kGroupWarps = kProdWarps / kGroups;
+constexpr int kInFlight = 4;
+static_assert(kGroupWarps == 4, "the blocks below are laid out for 128 threads");
 
-// Operand views of one tile's K slab for the producers.
 template <typename TIn>
-struct SlabSrc {
-  const TIn* a;
-  const TIn* b;
-  long long lda, ldb;
-  bool a_kc, b_kc;  // stored contiguous along K
-  int m, n, k;      // valid rows of A, of B, and K
-  int m0, n0, bn;
+__device__ __forceinline__ uint32_t ld_bits(const TIn* p) {
+  if constexpr (sizeof(TIn) == 4) return __ldg(reinterpret_cast<const unsigned int*>(p));
+  else return __ldg(reinterpret_cast<const unsigned short*>(p));
+}
+
+// One operand of a tile as a producer thread sees it.
+template <typename TIn>
+struct Operand {
+  const TIn* p;        // this thread's first value of block 0 of the slab at hand
+  long long s0, s1;    // from value 2i to 2i + 1, from 2i to 2i + 2
+  long long block;     // from a block to the next
+  int rows;            // rows of the tile inside the operand
+  uint32_t dst;        // byte offset of this thread's part of block 0 in the stage
+  bool along_k;
+
+  __device__ __forceinline__ void init(const void* x, long long ld, bool along_k_, int row0, int rows_, int tid) {
+    const int w = tid >> 5, lane = tid & 31;
+    along_k = along_k_;
+    rows = rows_;
+    const TIn* base = static_cast<const TIn*>(x);
+    if (along_k) {
+      const int kp = lane & 15;
+      p = base + (size_t)(row0 + 8 * w + (lane >> 4)) * ld + 2 * kp;
+      s0 = 1;
+      block = 32 * ld;
+      dst = (uint32_t)(w * 512 + (lane >> 4) * 64 + (kp & 3) * 4 + ((kp >> 2) << 4));
+    } else {
+      p = base + row0 + lane + (size_t)(8 * w) * ld;
+      s0 = ld;
+      block = 32;
+      dst = (uint32_t)((lane >> 3) * 512 + (lane & 7) * 64 + ((w ^ ((lane >> 1) & 3)) << 4));
+    }
+    s1 = 2 * ld;
+  }
+  // Values of block b that are inside: bit j for value j, `left` K values remain.
+  __device__ __forceinline__ unsigned inside(int b, int left, int tid) const {
+    const int w = tid >> 5, lane = tid & 31;
+    if (along_k) {
+      const int dr = rows - (32 * b + 8 * w + (lane >> 4)), dk = left - 2 * (lane & 15);
+      const unsigned in_rows = dr <= 0 ? 0u : dr >= 7 ? 0xffu : (1u << (((dr + 1) >> 1) * 2)) - 1u;
+      return in_rows & (dk >= 2 ? 0xffu : dk == 1 ? 0x55u : 0u);
+    }
+    const int dk = left - 8 * w;
+    return 32 * b + lane >= rows || dk <= 0 ? 0u : dk >= 8 ? 0xffu : (1u << dk) - 1u;
+  }
+  // Loads the thread's 8 values (bits) of block b; zeros outside the operand.
+  __device__ __forceinline__ void load(int b, int left, int tid, uint32_t (&v)[8]) const {
+    const TIn* q = p + b * block;
+    if (left >= kTK && 32 * b + 32 <= rows) {
+#pragma unroll
+      for (int j = 0; j < 8; j += 2, q += s1) {
+        v[j] = ld_bits(q);
+        v[j + 1] = ld_bits(q + s0);
+      }
+    } else {
+      const unsigned ok = inside(b, left, tid);
+#pragma unroll
+      for (int j = 0; j < 8; j += 2, q += s1) {
+        v[j] = v[j + 1] = 0u;
+        if (ok & (1u << j)) v[j] = ld_bits(q);
+        if (ok & (2u << j)) v[j + 1] = ld_bits(q + s0);
+      }
+    }
+  }
 };
 
-// Byte offset of element (row r, K position kk) of a slab tile in the
-// 64-byte-swizzled K-major layout (rows of 32 bf16, 8-row / 512-byte atoms,
-// 16-byte chunk c of row r at chunk c ^ ((r >> 1) & 3)).
-__device__ __forceinline__ uint32_t sw64_offset(int r, int kk) {
-  return (uint32_t)(r >> 3) * 512u + (uint32_t)(r & 7) * 64u + (uint32_t)((((kk >> 3) ^ ((r >> 1) & 3)) << 4) +
-                                                                           (kk & 7) * 2);
-}
-
-// Eight consecutive floats p[0..8), with two 16-byte loads when p is 16-byte
-// aligned (bf16 operands are staged raw by load_share_bf16 instead).
-__device__ __forceinline__ void ld8(const float* p, float* v) {
-  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-    const float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __ldg(p + j);
-  }
-}
-// Item e of an operand tile: 8 consecutive K values of one row.  Along K the
-// items run row-major (4 per row: lanes on the chunks of 8 consecutive rows,
-// each item one contiguous 16- or 32-byte segment); along the rows they run
-// chunk-major (lanes on consecutive rows, each of the 8 loads one coalesced
-// row segment).
-__device__ __forceinline__ void item_rc(bool kc, int e, int rows, int& r, int& c) {
-  if (kc) {
-    r = e >> 2;
-    c = e & 3;
-  } else {
-    r = e % rows;
-    c = e / rows;
-  }
-}
-
-// Loads one operand's share of a 32-deep slab for this producer thread into
-// v[0 .. kVals): rows [row0, row0 + rows) of an operand stored contiguous
-// along K (element (r, k) at X[k + r ld]) or along the rows (X[r + k ld]),
-// one item of 8 K values per 8 entries of v.  Everything outside R x Kd (and
-// rows past `rows`) reads as zero.
-template <typename TIn, int kVals>
-__device__ __forceinline__ void load_share(const TIn* __restrict__ X, long long ld, bool kc, int R, int Kd,
-                                           int row0, int rows, int k0, int ptid, float (&v)[kVals]) {
-  constexpr int kPT = 32 * kProdWarps;
-#pragma unroll
-  for (int i = 0; i < kVals; ++i) v[i] = 0.f;
-#pragma unroll
-  for (int it = 0; it < kVals / 8; ++it) {
-    const int e = ptid + it * kPT;
-    if (e >= rows * 4) continue;
-    int r, c;
-    item_rc(kc, e, rows, r, c);
-    const int gr = row0 + r, gk = k0 + 8 * c;
-    if (gr >= R) continue;
-    if (kc) {
-      const TIn* p = X + (size_t)gr * ld + gk;
-      if (gk + 8 <= Kd) {
-        ld8(p, &v[it * 8]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (gk + j < Kd) v[it * 8 + j] = ld_val<TIn>(p + j);
-      }
-    } else {
-      const TIn* p = X + gr + (size_t)gk * ld;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (gk + j < Kd) v[it * 8 + j] = ld_val<TIn>(p + (size_t)j * ld);
-    }
-  }
-}
-
-// Converts and stores what load_share loaded: NPC bf16 pieces of each value,
-// one 16-byte store per item and piece at dst + pc * piece_bytes.
-template <int NPC, int kVals>
-__device__ __forceinline__ void store_share(uint8_t* dst, uint32_t piece_bytes, bool kc, int rows, int ptid,
-                                            const float (&v)[kVals]) {
-  constexpr int kPT = 32 * kProdWarps;
-#pragma unroll
-  for (int it = 0; it < kVals / 8; ++it) {
-    const int e = ptid + it * kPT;
-    if (e >= rows * 4) continue;
-    int r, c;
-    item_rc(kc, e, rows, r, c);
-    __align__(16) __nv_bfloat16 q[NPC][8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const __nv_bfloat16 h0 = __float2bfloat16_rn(v[it * 8 + j]);
-      q[0][j] = h0;
-      if constexpr (NPC == 2) q[1][j] = __float2bfloat16_rn(v[it * 8 + j] - __bfloat162float(h0));
-    }
-    const uint32_t off = sw64_offset(r, 8 * c);
-#pragma unroll
-    for (int pc = 0; pc < NPC; ++pc)
-      *reinterpret_cast<uint4*>(dst + pc * piece_bytes + off) = *reinterpret_cast<const uint4*>(q[pc]);
-  }
-}
-
-// bf16 inputs need no conversion: their bits go to shared memory as loaded.
-// Loads one operand's share of a slab as packed bf16 pairs (w[it * 4 + h] =
-// K values 2h and 2h + 1 of item it), with the items of load_share; zero
-// bits (+0.0) outside R x Kd.
-template <int kItems>
-__device__ __forceinline__ void load_share_bf16(const __nv_bfloat16* __restrict__ X, long long ld, bool kc, int R,
-                                                int Kd, int row0, int rows, int k0, int ptid,
-                                                uint32_t (&w)[4 * kItems]) {
-  constexpr int kPT = 32 * kProdWarps;
-  const unsigned short* Xs = reinterpret_cast<const unsigned short*>(X);
-#pragma unroll
-  for (int i = 0; i < 4 * kItems; ++i) w[i] = 0u;
-#pragma unroll
-  for (int it = 0; it < kItems; ++it) {
-    const int e = ptid + it * kPT;
-    if (e >= rows * 4) continue;
-    int r, c;
-    item_rc(kc, e, rows, r, c);
-    const int gr = row0 + r, gk = k0 + 8 * c;
-    if (gr >= R) continue;
-    unsigned short h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (kc) {
-      const unsigned short* p = Xs + (size_t)gr * ld + gk;
-      if (gk + 8 <= Kd && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
-        w[it * 4 + 0] = u.x;
-        w[it * 4 + 1] = u.y;
-        w[it * 4 + 2] = u.z;
-        w[it * 4 + 3] = u.w;
-        continue;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (gk + j < Kd) h[j] = __ldg(p + j);
-    } else {
-      const unsigned short* p = Xs + gr + (size_t)gk * ld;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (gk + j < Kd) h[j] = __ldg(p + (size_t)j * ld);
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) w[it * 4 + j] = (uint32_t)h[2 * j] | ((uint32_t)h[2 * j + 1] << 16);
-  }
-}
-
-template <int kItems>
-__device__ __forceinline__ void store_share_bf16(uint8_t* dst, bool kc, int rows, int ptid,
-                                                 const uint32_t (&w)[4 * kItems]) {
-  constexpr int kPT = 32 * kProdWarps;
-#pragma unroll
-  for (int it = 0; it < kItems; ++it) {
-    const int e = ptid + it * kPT;
-    if (e >= rows * 4) continue;
-    int r, c;
-    item_rc(kc, e, rows, r, c);
-    *reinterpret_cast<uint4*>(dst + sw64_offset(r, 8 * c)) =
-        make_uint4(w[it * 4], w[it * 4 + 1], w[it * 4 + 2], w[it * 4 + 3]);
-  }
-}
-
-// Stages one 32-deep K slab of a tile: A rows [m0, m0 + 128) and B rows
-// [n0, n0 + bn) as NPC bf16 piece tiles, A pieces at st + i * kAPieceBytes
-// and B pieces after them, 64-byte swizzled.  Every load of the thread's share
-// of both operands is issued before any value is converted, so a slab costs
-// one memory round trip.
+// Two values as packed bf16 pieces (fp32: a = a0 + a1 + r; bf16: their bits).
 template <typename TIn, int NPC>
-__device__ __forceinline__ void stage_slab(const SlabSrc<TIn>& src, int k0, uint8_t* st, int ptid) {
-  constexpr int kAVals = kTM / kProdWarps;       // 8: one item of 8 K values per producer thread
-  constexpr int kBVals = kMaxBN / kProdWarps;    // 16: two items
-  if constexpr (std::is_same<TIn, __nv_bfloat16>::value) {
-    uint32_t wa[kAVals / 2], wb[kBVals / 2];
-    load_share_bf16<kAVals / 8>(src.a, src.lda, src.a_kc, src.m, src.k, src.m0, kTM, k0, ptid, wa);
-    load_share_bf16<kBVals / 8>(src.b, src.ldb, src.b_kc, src.n, src.k, src.n0, src.bn, k0, ptid, wb);
-    store_share_bf16<kAVals / 8>(st, src.a_kc, kTM, ptid, wa);
-    store_share_bf16<kBVals / 8>(st + kAPieceBytes, src.b_kc, src.bn, ptid, wb);
+__device__ __forceinline__ void pieces(uint32_t a, uint32_t b, uint32_t (&q)[NPC]) {
+  if constexpr (sizeof(TIn) == 2) {
+    q[0] = a | (b << 16);
   } else {
-    float va[kAVals], vb[kBVals];
-    load_share<TIn, kAVals>(src.a, src.lda, src.a_kc, src.m, src.k, src.m0, kTM, k0, ptid, va);
-    load_share<TIn, kBVals>(src.b, src.ldb, src.b_kc, src.n, src.k, src.n0, src.bn, k0, ptid, vb);
-    store_share<NPC, kAVals>(st, kAPieceBytes, src.a_kc, kTM, ptid, va);
-    store_share<NPC, kBVals>(st + NPC * kAPieceBytes, kBPieceBytes, src.b_kc, src.bn, ptid, vb);
+    const float fa = __uint_as_float(a), fb = __uint_as_float(b);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(fa, fb);
+    q[0] = *reinterpret_cast<const uint32_t*>(&h);
+    const __nv_bfloat162 l =
+        __floats2bfloat162_rn(fa - __uint_as_float(q[0] << 16), fb - __uint_as_float(q[0] & 0xffff0000u));
+    q[NPC - 1] = *reinterpret_cast<const uint32_t*>(&l);
+  }
+}
+
+// Writes a block's values into the 64-byte-swizzled K-major tile (rows of 32
+// bf16, 8-row / 512-byte atoms, 16-byte chunk c of row r at chunk c ^ ((r >> 1)
+// & 3)); d: the thread's place in the block, piece i at d + i * piece_bytes.
+template <typename TIn, int NPC>
+__device__ __forceinline__ void store_block(bool along_k, uint8_t* d, uint32_t piece_bytes, const uint32_t (&v)[8]) {
+  uint32_t q[4][NPC];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) pieces<TIn, NPC>(v[2 * h], v[2 * h + 1], q[h]);
+  if (along_k) {  // rows 2 apart: 128 bytes on, the chunk's low bits flipped
+    const uint32_t chunk = tc::smem_u32(d) & 0x30u;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      uint8_t* da = d + (int)((chunk ^ (a << 4)) - chunk) + a * 128;
+#pragma unroll
+      for (int i = 0; i < NPC; ++i) *reinterpret_cast<uint32_t*>(da + i * piece_bytes) = q[a][i];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NPC; ++i)
+      *reinterpret_cast<uint4*>(d + i * piece_bytes) = make_uint4(q[0][i], q[1][i], q[2][i], q[3][i]);
   }
 }
 
@@ -386,7 +367,7 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      tc::mbar_init(&full_bar[s], kProdWarps);
+      tc::mbar_init(&full_bar[s], 2 * kGroupWarps);
       tc::mbar_init(&empty_bar[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -414,92 +395,128 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
     atomicOr(status, kStatusTimeout);
     atomicExch(&abort_flag, 1);
   };
-  // Consumer side of the tile queue: the info of the j-th tile of this CTA.
-  // A whole warp calls it (one arrival per warp), or a single thread with
-  // single == true.
-  auto next_tile = [&](int j, TileInfo& ti, bool single) -> bool {
+  // Consumer side of the tile queue: the j-th tile of this CTA, which stays valid
+  // until release_tile(j) (one arrival per consumer warp).
+  auto next_tile = [&](int j) -> const TileInfo* {
     const int q = j % kQueue;
     if (!tc::mbar_wait(&tq_full[q], (j / kQueue) & 1, limit_ns)) {
       give_up();
-      return false;
+      return nullptr;
     }
-    ti = tq[q];
-    if (!single) __syncwarp();
-    if (single || lane == 0) tc::mbar_arrive(&tq_empty[q]);
-    return ti.inst >= 0 && !*(volatile int*)&abort_flag;
+    return tq[q].more && !*(volatile int*)&abort_flag ? &tq[q] : nullptr;
   };
+  auto release_tile = [&](int j) { tc::mbar_arrive(&tq_empty[j % kQueue]); };
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---- scheduler ----
-      const long long total = prefix[count];
-      for (int j = 0;; ++j) {
-        const int q = j % kQueue;
-        if (j >= kQueue && !tc::mbar_wait(&tq_empty[q], ((j / kQueue) - 1) & 1, limit_ns)) {
-          give_up();
-          break;
-        }
-        TileInfo ti{-1, 0, 0, 0, 0};
-        const long long t = *(volatile int*)&abort_flag ? total : (long long)atomicAdd(tile_counter, 1ull);
+    // ---- scheduler: kBatch tiles at a time, 8 lanes each ----
+    const long long total = prefix[count];
+    // fewer at a time where each CTA gets a few only, down to one
+    const int batch = (int)max(1ll, min((long long)kBatch, total / (4 * (long long)gridDim.x)));
+    const int g = lane >> 3, sub = lane & 7;
+    for (int j0 = 0;; j0 += batch) {
+      const int j = j0 + g, q = j % kQueue;
+      bool ok = true;
+      if (sub == 0 && j >= kQueue && g < batch) ok = tc::mbar_wait(&tq_empty[q], ((j / kQueue) - 1) & 1, limit_ns);
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) give_up();
+        break;
+      }
+      long long t = 0;
+      if (lane == 0) t = *(volatile int*)&abort_flag ? total : (long long)atomicAdd(tile_counter, (unsigned long long)batch);
+      t = __shfl_sync(0xffffffffu, t, 0) + g;
+      // last position with prefix <= t, an 8-way step at a time
+      int lo = 0, hi = t < total ? count - 1 : 0;
+      while (__any_sync(0xffffffffu, lo < hi)) {
+        const int step = (hi - lo + 8) / 8, at = lo + (sub + 1) * step;
+        const bool le = at <= hi && prefix[at] <= t;
+        const int c = __popc((__ballot_sync(0xffffffffu, le) >> (8 * g)) & 0xffu);
+        lo += c * step;
+        hi = min(hi, lo + step - 1);
+      }
+      if (sub == 0 && g < batch) {
+        TileInfo ti{};
         if (t < total) {
-          int lo = 0, hi = count - 1;  // last position with prefix <= t
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (prefix[mid] <= t) lo = mid; else hi = mid - 1;
-          }
-          const int inst = order[lo];
-          const coral_sgemm_problem_t p = probs[inst];
-          const int bn = bn_pos[lo];
+          ti.p = probs[order[lo]];
+          ti.more = 1;
+          ti.bn = bn_pos[lo];
           const long long local = t - prefix[lo];
-          const int mt = (p.m + kTM - 1) / kTM;
-          ti.inst = inst;
-          ti.bn = bn;
+          const int mt = (ti.p.m + kTM - 1) / kTM;
           ti.m0 = (int)(local % mt) * kTM;
-          ti.n0 = (int)(local / mt) * bn;
-          ti.nslabs = (p.alpha == 0.f || p.k <= 0) ? 0 : (p.k + kTK - 1) / kTK;
+          ti.n0 = (int)(local / mt) * ti.bn;
+          ti.nslabs = (ti.p.alpha == 0.f || ti.p.k <= 0) ? 0 : (ti.p.k + kTK - 1) / kTK;
         }
         tq[q] = ti;
         tc::mbar_arrive(&tq_full[q]);
-        if (ti.inst < 0) break;
       }
+      if (__shfl_sync(0xffffffffu, t, 8 * (batch - 1)) >= total) break;  // the batch held an end mark
     }
   } else if (warp < kMmaWarp) {
-    // ---- producers ----
-    const int ptid = threadIdx.x - 32;
-    int it = 0;
-    TileInfo ti;
-    for (int j = 0; next_tile(j, ti, false); ++j) {
-      if (ti.nslabs == 0) continue;
-      const coral_sgemm_problem_t p = probs[ti.inst];
-      const SlabSrc<TIn> src{static_cast<const TIn*>(p.a), static_cast<const TIn*>(p.b), p.lda, p.ldb,
-                             p.op_a != CORAL_NO_TRANSPOSE, p.op_b == CORAL_NO_TRANSPOSE, p.m, p.n, p.k,
-                             ti.m0, ti.n0, ti.bn};
-      bool stop = false;
-      for (int kb = 0; kb < ti.nslabs; ++kb, ++it) {
-        const int s = it % S;
-        if (it >= S && !tc::mbar_wait(&empty_bar[s], ((it / S) - 1) & 1, limit_ns)) {
-          give_up();
-          stop = true;
-          break;
-        }
-        uint8_t* st = smem + (size_t)s * kStage;
-        stage_slab<TIn, NPC>(src, kb * kTK, st, ptid);
-        tc::fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&full_bar[s]);
+    // ---- producers: groups 0 and 1 stage A, 2 and 3 stage B, of even and odd slabs ----
+    const int ptid = threadIdx.x - 32, group = ptid / (32 * kGroupWarps), tid = ptid % (32 * kGroupWarps);
+    const bool is_a = group < 2;
+    const uint32_t piece_bytes = is_a ? kAPieceBytes : kBPieceBytes;
+    int it0 = 0;  // running number of the tile's first slab
+    bool stop = false;
+    const TileInfo* tp;
+    for (int j = 0; !stop && (tp = next_tile(j)); ++j) {
+      const TileInfo& ti = *tp;
+      const coral_sgemm_problem_t& p = ti.p;
+      // C is read in the epilogue, a column at a time: bring it into L2 now
+      if (p.beta != 0.f && !(p.beta == 1.f && ti.nslabs == 0)) {
+        const int cols = min(ti.bn, p.n - ti.n0), row = ti.m0 + (ptid & 3) * 32;
+        if (row < p.m)
+          for (int c = ptid >> 2; c < cols; c += 8 * kProdWarps)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.c + row + (size_t)(ti.n0 + c) * p.ldc));
       }
-      if (stop) break;
+      const int nslabs = ti.nslabs, kd = p.k;
+      if (nslabs) {
+        Operand<TIn> o;
+        if (is_a)
+          o.init(p.a, p.lda, p.op_a != CORAL_NO_TRANSPOSE, ti.m0, min(kTM, p.m - ti.m0), tid);
+        else
+          o.init(p.b, p.ldb, p.op_b == CORAL_NO_TRANSPOSE, ti.n0, min(ti.bn, p.n - ti.n0), tid);
+        const long long slab = o.along_k ? kTK : kTK * (o.s1 >> 1);
+        const int nb = (o.rows + 31) >> 5;
+        int kb = (group ^ it0) & 1;
+        o.p += kb * slab;
+        for (; kb < nslabs; kb += 2, o.p += 2 * slab) {
+          const int it = it0 + kb, s = it % S, left = kd - kb * kTK;
+          uint8_t* st = smem + (size_t)s * kStage + (is_a ? 0 : NPC * kAPieceBytes) + o.dst;
+          for (int b0 = 0; b0 < nb; b0 += kInFlight) {
+            uint32_t v[kInFlight][8];
+#pragma unroll
+            for (int u = 0; u < kInFlight; ++u)
+              if (b0 + u < nb) o.load(b0 + u, left, tid, v[u]);
+            if (b0 == 0 && it >= S && !tc::mbar_wait(&empty_bar[s], ((it / S) - 1) & 1, limit_ns)) {
+              give_up();
+              stop = true;
+              break;
+            }
+#pragma unroll
+            for (int u = 0; u < kInFlight; ++u)
+              if (b0 + u < nb) store_block<TIn, NPC>(o.along_k, st + (b0 + u) * 2048, piece_bytes, v[u]);
+          }
+          if (stop) break;
+          tc::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&full_bar[s]);
+        }
+        it0 += nslabs;
+      }
+      __syncwarp();
+      if (lane == 0) release_tile(j);
     }
   } else if (warp == kMmaWarp) {
     if (lane == 0) {
       // ---- MMA issuer ----
       int it = 0, gc = 0;
       bool stop = false;
-      TileInfo ti;
-      for (int j = 0; !stop && next_tile(j, ti, true); ++j) {
-        if (ti.nslabs == 0) continue;
-        const uint32_t idesc = tc::idesc_bf16_f32(kTM, ti.bn);
-        const int chunks = (ti.nslabs + kChunkSlabs - 1) / kChunkSlabs;
+      const TileInfo* tp;
+      for (int j = 0; !stop && (tp = next_tile(j)); ++j) {
+        const int nslabs = tp->nslabs;
+        const uint32_t idesc = tc::idesc_bf16_f32(kTM, tp->bn);
+        release_tile(j);
+        const int chunks = (nslabs + kChunkSlabs - 1) / kChunkSlabs;
         for (int c = 0; c < chunks && !stop; ++c, ++gc) {
           const int b = gc & 1;
           if (gc >= 2 && !tc::mbar_wait(&acc_empty[b], ((gc >> 1) - 1) & 1, limit_ns)) {
@@ -509,7 +526,7 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
           }
           tc::tc_fence_after();
           const uint32_t acc = tmem + b * kMaxBN;
-          const int kb0 = c * kChunkSlabs, kb1 = min(ti.nslabs, kb0 + kChunkSlabs);
+          const int kb0 = c * kChunkSlabs, kb1 = min(nslabs, kb0 + kChunkSlabs);
           for (int kb = kb0; kb < kb1; ++kb, ++it) {
             const int s = it % S;
             if (!tc::mbar_wait(&full_bar[s], (it / S) & 1, limit_ns)) {
@@ -548,65 +565,89 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
     }
   } else {
     // ---- epilogue ----
-    const int quad = warp & 3;
+    const int quad = warp & 3, half = (warp - kEpiWarp0) >> 2;  // rows; every other group of 16 columns
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
     int gc = 0;
-    TileInfo ti;
-    for (int j = 0; next_tile(j, ti, false); ++j) {
-      const coral_sgemm_problem_t p = probs[ti.inst];
-      const int row = ti.m0 + quad * 32 + lane;
-      const bool beta0 = p.beta == 0.f, beta1 = p.beta == 1.f;
-      const int ncols = min(ti.bn, p.n - ti.n0);
-      float* crow = p.c + row;
-      if (ti.nslabs == 0) {  // scale-only (sgemm_nn.rs:29-45), 16 C loads before their stores
-        if (!beta1 && row < p.m)
-          for (int g = 0; g < ncols; g += 16) {
+    bool stop = false;
+    const TileInfo* tp;
+    for (int j = 0; !stop && (tp = next_tile(j)); ++j) {
+      const int m0 = tp->m0, n0 = tp->n0, nslabs = tp->nslabs, m = tp->p.m;
+      const int row = m0 + quad * 32 + lane;
+      const int ncols = min(tp->bn, tp->p.n - n0);
+      const float alpha = tp->p.alpha, beta = tp->p.beta;
+      const bool beta0 = beta == 0.f, beta1 = beta == 1.f;
+      const long long ldc = tp->p.ldc;
+      float* const crow = tp->p.c + row + (size_t)n0 * ldc;
+      __syncwarp();
+      if (lane == 0) release_tile(j);
+      if (nslabs == 0) {  // scale-only (sgemm_nn.rs:29-45), 16 C loads before their stores
+        if (!beta1 && row < m)
+          for (int g = 16 * half; g < ncols; g += 32) {
             float cv[16];
 #pragma unroll
             for (int jj = 0; jj < 16; ++jj)
-              cv[jj] = (!beta0 && g + jj < ncols) ? crow[(size_t)(ti.n0 + g + jj) * p.ldc] : 0.f;
+              cv[jj] = (!beta0 && g + jj < ncols) ? crow[(size_t)(g + jj) * ldc] : 0.f;
 #pragma unroll
             for (int jj = 0; jj < 16; ++jj)
-              if (g + jj < ncols) crow[(size_t)(ti.n0 + g + jj) * p.ldc] = beta0 ? 0.f : p.beta * cv[jj];
+              if (g + jj < ncols) crow[(size_t)(g + jj) * ldc] = beta0 ? 0.f : beta * cv[jj];
           }
         continue;
       }
-      const int chunks = (ti.nslabs + kChunkSlabs - 1) / kChunkSlabs;
-      bool stop = false;
+      const int chunks = (nslabs + kChunkSlabs - 1) / kChunkSlabs;
       for (int c = 0; c < chunks; ++c, ++gc) {
         const int b = gc & 1;
+        const bool in = row < m, read_c = (c > 0 || !beta0) && in;
+        const float keep = c > 0 ? 1.f : beta;  // factor of what C holds
+        float cv[16];
+        float* q = crow + (size_t)(16 * half) * ldc;
+        auto load_c = [&](const float* from, int cols) {  // up to 16 columns
+          if (!read_c) return;
+          if (cols >= 16) {
+#pragma unroll
+            for (int jj = 0; jj < 16; ++jj, from += ldc) cv[jj] = *from;
+          } else {
+#pragma unroll
+            for (int jj = 0; jj < 16; ++jj, from += ldc)
+              if (jj < cols) cv[jj] = *from;
+          }
+        };
+        // the first 16 columns of C on their way while the products finish
+        load_c(q, ncols - 16 * half);
         if (!tc::mbar_wait(&acc_full[b], (gc >> 1) & 1, limit_ns)) {
           give_up();
           stop = true;
           break;
         }
         tc::tc_fence_after();
-        const bool read_c = c > 0 || !beta0;
-        for (int col0 = 0; col0 < ncols; col0 += 16) {
-          // 16 accumulator columns, then every C load of them before any store
+        for (int col0 = 16 * half; col0 < ncols; col0 += 32) {
           uint32_t r[16];
           tc::tmem_ld16(tmem + b * kMaxBN + col0 + lane_base, r);
           tc::tmem_wait_ld();
-          if (row < p.m) {
-            const int lim = min(16, ncols - col0);
-            float cv[16];
+          float out[16];
 #pragma unroll
-            for (int jj = 0; jj < 16; ++jj)
-              cv[jj] = (read_c && jj < lim) ? crow[(size_t)(ti.n0 + col0 + jj) * p.ldc] : 0.f;
+          for (int jj = 0; jj < 16; ++jj) {
+            const float v = alpha * __uint_as_float(r[jj]);
+            out[jj] = keep == 1.f ? cv[jj] + v : keep == 0.f ? v : keep * cv[jj] + v;
+          }
+          // the next group's C before this group's stores
+          load_c(q + 32 * ldc, ncols - col0 - 32);
+          if (in) {
+            float* to = q;
+            if (ncols - col0 >= 16) {
 #pragma unroll
-            for (int jj = 0; jj < 16; ++jj) {
-              if (jj >= lim) break;
-              const float v = p.alpha * __uint_as_float(r[jj]);
-              crow[(size_t)(ti.n0 + col0 + jj) * p.ldc] =
-                  (c > 0 || beta1) ? cv[jj] + v : beta0 ? v : p.beta * cv[jj] + v;
+              for (int jj = 0; jj < 16; ++jj, to += ldc) *to = out[jj];
+            } else {
+#pragma unroll
+              for (int jj = 0; jj < 16; ++jj, to += ldc)
+                if (col0 + jj < ncols) *to = out[jj];
             }
           }
+          q += 32 * ldc;
         }
         tc::tc_fence_before();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&acc_empty[b]);
       }
-      if (stop) break;
     }
   }
   tc::tc_fence_before();
