@@ -77,6 +77,21 @@ bool encode_kmajor_map(CUtensorMap* map, const void* base, int elem_bytes, uint6
   return r == CUDA_SUCCESS;
 }
 
+bool encode_slices_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t slices,
+                       uint64_t row_stride, uint64_t slice_stride, uint32_t box_inner, uint32_t box_rows,
+                       uint32_t box_slices) {
+  auto fn = tmap_encode_fn();
+  if (!fn) return false;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_stride & 15) || (slice_stride & 15)) return false;
+  cuuint64_t dims[3] = {inner, rows, slices};
+  cuuint64_t strides[2] = {row_stride, slice_stride};
+  cuuint32_t box[3] = {box_inner, box_rows, box_slices};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 namespace {
 
 constexpr int kBM = 128;

@@ -10,13 +10,13 @@
 //      v = sum_p A_p 2^-7p + r with A_p = trunc(2^7 r_{p-1}) in [-127, 127]
 //      and |r| < 2^-7S: every step is exact in FP64.  Slices are stored
 //      K-major, int8, [S][rows][kp] (kp = k rounded up to 16 bytes).
-//   3. GEMM: for a 128 x 64 tile of C, the products A_p B_q^T with p + q <= S+1
-//      (S(S+1)/2 of them; the rest are below 2^-7(S+1)) are accumulated in
-//      INT32 in TMEM, one accumulator per anti-diagonal d = p + q, exactly as
-//      long as (#products on d) * 127^2 * kchunk < 2^31 -- K is cut into
-//      chunks that satisfy it.  After each chunk the epilogue warps convert
-//      each diagonal accumulator to FP64 and add 2^-7d times it to registers
-//      (exact scaling, one FP64 rounding per add).
+//   3. GEMM: for a 128 x 64 or 128 x 128 tile of C, the products A_p B_q^T with
+//      p + q <= S+1 (S(S+1)/2 of them; the rest are below 2^-7(S+1)) are
+//      accumulated in INT32 in TMEM, one accumulator per anti-diagonal d = p + q,
+//      exactly as long as (#products on d) * 127^2 * kchunk < 2^30 -- K is cut into
+//      chunks that satisfy it.  After each pass the epilogue warps combine the
+//      diagonals in 64-bit integers (exact) and add them to FP64 registers, one
+//      rounding per pass.
 //   4. Epilogue: C = alpha * 2^(e_i + f_j) * acc + beta * C in FP64 (beta == 0
 //      does not read C, as f64_edge / f32_edge.rs:37-58 do).
 // Complex operands (ZGEMM) use the same 4M folding as the split-BF16 CGEMM:
@@ -24,10 +24,15 @@
 // or, with the handle's complex mapping set to 3M, three real Ozaki GEMMs
 // combined as Re = T1 - T2, Im = T3 - T1 - T2 (zgemm_ozaki_3m).
 //
-// Pipeline: warp 0 lane 0 = TMA producer (2 stages of S slices of A and B,
-// 64-byte K slabs, 64-byte swizzle); warp 1 lane 0 = MMA issuer (kind::i8,
-// M=128, N=64, K=32 per instruction); warps 2-9 = epilogue.  All waits are
-// bounded and report through the handle's status word.
+// Pipeline: warp 0 lane 0 = TMA producer (two K slabs of 64 bytes in four slots,
+// 64-byte swizzle, 3-D maps over the slices); warp 1 = MMA issuer (kind::i8, M=128,
+// N=64 or 128, K=32 per instruction), converged so that descriptors stay in
+// uniform registers; warps 2-9 = epilogue.  All waits are bounded and report
+// through the handle's status word.
+//
+// Bound: the int8 tensor pipe under the power cap.  DGEMM NN 4096^3: 1.97 -> 1.37 ms
+// a call, the GEMM kernel 1.56 -> 1.18 ms (tensor pipe 56 -> 84% busy at 1.63 GHz);
+// the same with one barrier per slab, 128-column tiles and one lane issuing 1.20.
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -36,8 +41,7 @@
 namespace coral {
 namespace {
 
-constexpr int kOzBM = 128, kOzBN = 64, kOzBK = 64;  // BK in int8 elements (64 bytes)
-constexpr int kOzStages = 2;
+constexpr int kOzBM = 128, kOzBK = 64;  // BK in int8 elements (64 bytes)
 constexpr int kOzEpiWarps = 8;
 constexpr int kOzThreads = 64 + 32 * kOzEpiWarps;
 
@@ -120,48 +124,104 @@ coral_status_t launch_row_exponent(Handle* h, const T* X, size_t ld, int R, int 
 }
 
 // ---- 2. slicing ----------------------------------------------------------------
+// The digits of |a| 2^-ex to the base 128 are 7-bit fields of its mantissa,
+// shifted: taking them with integer operations gives what the loop
+// "r *= 128, t = trunc(r), r -= t" gives, without its 4 fp64 operations and
+// conversions per slice.  `low`: the lowest 28 bits (slices 4-7), `high`: the
+// 21 above (slices 1-3); the sign applies to every slice.
+struct SliceBits {
+  uint32_t high, low;
+  bool neg;
+};
+__device__ __forceinline__ SliceBits slice_bits(double a, int ex) {
+  long long bits = __double_as_longlong(a);
+  int field = (int)((bits >> 52) & 0x7ff);
+  SliceBits s{0u, 0u, bits < 0};
+  if (field == 0x7ff) {  // NaN slices to 0; an infinity as trunc and the int conversion leave it
+    if ((bits & 0xfffffffffffffll) == 0 && !s.neg) {
+      s.high = 1u << 14;
+      s.neg = true;
+    }
+    return s;
+  }
+  int e = field - 1022;  // frexp: |a| in [2^(e-1), 2^e)
+  if (field == 0) {      // zero or subnormal: scaled up exactly
+    bits = __double_as_longlong(a * 0x1p64);
+    field = (int)((bits >> 52) & 0x7ff);
+    if (field == 0) return s;
+    e = field - 1022 - 64;
+  }
+  const unsigned long long mant = ((unsigned long long)bits & 0xfffffffffffffull) | 0x10000000000000ull;
+  const int shift = min(max(4 + ex - e, 4), 63);  // ex >= e: the row's largest exponent
+  const unsigned long long m = mant >> shift;
+  s.high = (uint32_t)(m >> 28);
+  s.low = (uint32_t)m & 0xfffffffu;
+  return s;
+}
+__device__ __forceinline__ uint32_t slice_digit(const SliceBits& s, int p) {  // p = 0..6
+  return p < 3 ? (s.high >> (14 - 7 * p)) & 127u : (s.low >> (42 - 7 * p)) & 127u;
+}
 template <int S>
-__device__ __forceinline__ void slice_value(double a, int ex, int8_t (&s)[S]) {
-  double r = ldexp(a, -ex);  // |r| < 1
+__device__ __forceinline__ void slice_value(double a, int ex, int8_t (&out)[S]) {
+  static_assert(S == 7, "seven 7-bit slices of a 49-bit fixed-point value");
+  const SliceBits b = slice_bits(a, ex);
 #pragma unroll
   for (int p = 0; p < S; ++p) {
-    r *= 128.0;
-    const double t = trunc(r);
-    s[p] = (int8_t)(int)t;
-    r -= t;
+    const int d = (int)slice_digit(b, p);
+    out[p] = (int8_t)(b.neg ? -d : d);
   }
 }
 
-// Real: dst[p][row][l] for op(X) rows (K contiguous).
+// Real: dst[p][row][l] for op(X) rows (K contiguous).  A CTA slices 32 rows x
+// 128 K values through shared memory, 16 loads in flight per thread; a thread
+// writes 16 K values of a row, 16 bytes per slice (rows of kp bytes, a multiple
+// of 16).  Bound: HBM (8 B read, 7 B written per element); 4096^2: 70 ->
+// 50 us against the fp64 loop with byte stores (64 with words).
 template <int S, bool kKMajorSrc>
 __global__ void __launch_bounds__(256)
 k_slice_real(const double* __restrict__ X, size_t ld, int R, int Kd, const int* __restrict__ e,
              int8_t* __restrict__ dst, size_t kp, size_t piece) {
-  __shared__ double tile[32][33];
-  const int r0 = blockIdx.y * 32, l0 = blockIdx.x * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  // element (r, l) at r * kPitch + l + l / 16: no bank conflicts either way
+  constexpr int kRows = 32, kDepth = 128, kPitch = 137, kPer = kRows * kDepth / 256;
+  __shared__ double tile[kRows * kPitch];
+  const int r0 = blockIdx.y * kRows, l0 = blockIdx.x * kDepth;
+  const int g = threadIdx.x & 7, row = threadIdx.x >> 3, r_out = r0 + row, l_out = l0 + 16 * g;
+  const int ex = r_out < R ? e[r_out] : 0;
+  double v[kPer];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    if (kKMajorSrc) {
-      int r = r0 + ty + 8 * q, l = l0 + tx;
-      tile[ty + 8 * q][tx] = (r < R && l < Kd) ? __ldg(X + l + (size_t)r * ld) : 0.0;
-    } else {
-      int l = l0 + ty + 8 * q, r = r0 + tx;
-      tile[tx][ty + 8 * q] = (r < R && l < Kd) ? __ldg(X + r + (size_t)l * ld) : 0.0;
-    }
+  for (int q = 0; q < kPer; ++q) {
+    const int i = threadIdx.x + 256 * q;
+    const int r = r0 + (kKMajorSrc ? i / kDepth : i % kRows), l = l0 + (kKMajorSrc ? i % kDepth : i / kRows);
+    v[q] = r < R && l < Kd ? __ldg(kKMajorSrc ? X + l + (size_t)r * ld : X + r + (size_t)l * ld) : 0.0;
+  }
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int i = threadIdx.x + 256 * q, l = kKMajorSrc ? i % kDepth : i / kRows;
+    tile[(kKMajorSrc ? i / kDepth : i % kRows) * kPitch + l + l / 16] = v[q];
   }
   __syncthreads();
+  if (r_out >= R || l_out >= (int)kp) return;
+  uint32_t w[S][4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int r = r0 + ty + 8 * q, l = l0 + tx;
-    if (r < R && l < (int)kp) {
-      int8_t s[S];
-      slice_value<S>(tile[ty + 8 * q][tx], e[r], s);
-      const size_t o = (size_t)r * kp + l;
+  for (int a = 0; a < 4; ++a) {
+    uint32_t negs = 0u;
 #pragma unroll
-      for (int p = 0; p < S; ++p) dst[p * piece + o] = s[p];
+    for (int b = 0; b < 4; ++b) {
+      const SliceBits s = slice_bits(tile[row * kPitch + 17 * g + 4 * a + b], ex);
+#pragma unroll
+      for (int p = 0; p < S; ++p) w[p][a] = (b ? w[p][a] : 0u) | slice_digit(s, p) << (8 * b);
+      if (s.neg) negs |= 0xffu << (8 * b);
+    }
+#pragma unroll
+    for (int p = 0; p < S; ++p) {  // bytes are 0..127: 0x80 - d, top bit flipped, is -d
+      const uint32_t minus = (0x80808080u - w[p][a]) ^ 0x80808080u;
+      w[p][a] = (w[p][a] & ~negs) | (minus & negs);
     }
   }
+  int8_t* o = dst + (size_t)r_out * kp + l_out;
+#pragma unroll
+  for (int p = 0; p < S; ++p)
+    *reinterpret_cast<uint4*>(o + p * piece) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
 }
 
 // Complex, 4M layout (see k_split_cplx in gemm_split.cu): A rows [Re | Im];
@@ -217,8 +277,8 @@ k_slice_cplx(const double2* __restrict__ X, size_t ld, int R, int Kd, bool conj,
 
 // ---- 3./4. integer GEMM and FP64 recombination -----------------------------------
 struct OzMaps {
-  CUtensorMap a[8];
-  CUtensorMap b[8];
+  CUtensorMap a[2];  // boxes of 3 and of 4 slices
+  CUtensorMap b[2];
 };
 
 struct OzEpi {
@@ -242,30 +302,117 @@ __device__ __forceinline__ void oz_tile_coords(int tile, int m_tiles, int n_tile
   nt = within / gsz;
 }
 
-template <int S>
+// How a tile of BN columns goes through the diagonals d = p + q = 2..8, with one
+// BN-column accumulator each in the 512 TMEM columns: BN = 64 takes all seven in
+// one pass over K; BN = 128 takes d = 5..8 (22 of the 28 products, all slices),
+// then d = 2..4 (6 products, slices 1-3).  An int8 product of 128 x 64 x 32 reads
+// as many bytes of shared memory per cycle as there are (48 cycles, 36 with A
+// kept in the collector, 32 at the tensor core's peak); one of 128 x 128 x 32 runs
+// at its peak of 64.  The wide tile takes more time to drain and write, and half
+// as many tiles fill the last wave worse, so run_ozaki_gemm weighs both.
+//
+// The ring holds two K slabs, each in two slots: "high" (A_4..A_7, B_1..B_4) and
+// "low" (A_1..A_3, B_5..B_7).  The products of a slab run as high x high, low A x
+// high B, low x low, so a slab starts when its high slot has arrived, the low
+// one is needed 10 products later, and the high one is free again 6 (BN = 64:
+// 12) before the end: each load has more time than with one barrier per slab
+// (80% of the tensor peak).  One barrier per slice had more still, but its
+// single issuing lane could not keep up (76%).  In the second pass of BN = 128 a
+// slot holds slices 1-3 of a whole slab.  A 3-D tensor map loads a slot's slices
+// of one operand at once.
+enum OzPart { kOzHighHigh, kOzLowHigh, kOzLowLow, kOzSecondPass };
+template <int BN>
+struct OzPlan {
+  static constexpr int kPasses = BN == 64 ? 1 : 2;
+  static constexpr int kLo = BN == 64 ? 2 : 5;       // first pass: d = kLo..8
+  static constexpr int kSlabCycles = 56 * (BN == 64 ? 36 : 64);           // a K slab's 2 x 28 products
+  static constexpr int kTileCycles = BN == 64 ? 16000 : 40000;            // drain and epilogue of a tile
+  static constexpr uint32_t kATile = kOzBM * kOzBK, kBTile = BN * kOzBK;  // bytes per slice
+  static constexpr uint32_t kHigh = 4 * (kATile + kBTile), kLow = 3 * (kATile + kBTile);
+  static constexpr int kSlots = 4;                                        // high, low, high, low
+  __device__ static constexpr uint32_t offset(int slot) { return (slot >> 1) * (kHigh + kLow) + (slot & 1) * kHigh; }
+};
+
+// The products of one part of a slab: A_p at a + (p - 1 from the part's first) etc.,
+// as low descriptor words.  `first`: the slab starts the accumulators.
+template <int BN, int kPart>
+__device__ __forceinline__ void oz_issue(uint32_t a, uint32_t b, uint32_t hi, uint32_t tmem, bool first) {
+  using P = OzPlan<BN>;
+  constexpr uint32_t kIdesc = tc::idesc_s8_s32(kOzBM, BN);
+  constexpr int lo = kPart == kOzSecondPass ? 2 : P::kLo, top = kPart == kOzSecondPass ? 4 : 8;
+  constexpr int p0 = kPart == kOzHighHigh ? 4 : 1, p1 = kPart == kOzHighHigh ? 7 : 3;
+  constexpr int b0 = kPart == kOzLowLow ? 5 : 1, b1 = kPart == kOzLowLow ? 7 : kPart == kOzSecondPass ? 3 : 4;
+#pragma unroll
+  for (int p = p0; p <= p1; ++p) {
+    const int q0 = lo - p > b0 ? lo - p : b0, q1 = top - p < b1 ? top - p : b1;
+#pragma unroll
+    for (int kk = 0; kk < kOzBK / 32; ++kk) {
+      const uint32_t ad = a + (uint32_t)(p - p0) * (P::kATile >> 4) + kk * 2;
+#pragma unroll
+      for (int q = q0; q <= q1; ++q) {
+        const uint32_t acc = tmem + (p + q - lo) * BN;
+        const uint32_t bd = b + (uint32_t)(q - b0) * (P::kBTile >> 4) + kk * 2;
+        // which products meet their diagonal first: A_4's (d = 5..8), then A_1's (d = 2..4)
+        const bool opens = kk == 0 && (kPart == kOzHighHigh ? p == 4 : kPart == kOzLowLow ? false : p == 1 && p + q <= 4);
+        const uint32_t accum = opens && first ? 0u : 1u;
+        // A_p stays in the collector over its products
+        if (q0 == q1) tc::mma_i8_ca<tc::kCollectNone>(acc, ad, bd, hi, kIdesc, accum);
+        else if (q == q0) tc::mma_i8_ca<tc::kCollectFill>(acc, ad, bd, hi, kIdesc, accum);
+        else if (q == q1) tc::mma_i8_ca<tc::kCollectLastUse>(acc, ad, bd, hi, kIdesc, accum);
+        else tc::mma_i8_ca<tc::kCollectUse>(acc, ad, bd, hi, kIdesc, accum);
+      }
+    }
+  }
+}
+
+// sum[j] += 2^(-7 hi) * (diagonals lo..hi of column j, each 2^7 below the last):
+// the integer combination is exact in 64 bits (below 2^51, see oz_chunk_slabs),
+// so a pass costs one fp64 conversion -- an addition to 1.5 * 2^52 -- and one
+// multiply-add per element, where converting each diagonal took seven.
+template <int kLo, int kHi, int BN, int kCols>
+__device__ __forceinline__ void oz_drain(uint32_t acc, double (&sum)[kCols]) {
+  constexpr int kD = kHi - kLo + 1;
+  constexpr double kScale = 1.0 / (double)(1ull << (7 * kHi));
+#pragma unroll
+  for (int c0 = 0; c0 < kCols; c0 += 8) {
+    uint32_t r[kD][8];
+#pragma unroll
+    for (int d = 0; d < kD; ++d) tc::tmem_ld8(acc + d * BN + c0, r[d]);
+    tc::tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      long long x = (int)r[0][j];
+#pragma unroll
+      for (int d = 1; d < kD; ++d) x = x * 128 + (int)r[d][j];
+      const double v = __longlong_as_double(x + 0x4338000000000000ll) - 6755399441055744.0;
+      sum[c0 + j] = fma(v, kScale, sum[c0 + j]);
+    }
+  }
+}
+
+template <int S, int BN>
 __global__ void __launch_bounds__(kOzThreads, 1)
 k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_tiles,
              int chunk_kb, OzEpi ep, unsigned* status, uint64_t limit_ns) {
-  constexpr uint32_t kATile = kOzBM * kOzBK;  // bytes
-  constexpr uint32_t kBTile = kOzBN * kOzBK;
-  constexpr uint32_t kStageBytes = S * (kATile + kBTile);
-  constexpr uint32_t kIdesc = tc::idesc_s8_s32(kOzBM, kOzBN);
-  constexpr int kCols = kOzBN / 2;  // columns per epilogue thread
+  static_assert(S == 7, "the passes are laid out for seven slices");
+  using P = OzPlan<BN>;
+  constexpr uint32_t kATile = P::kATile, kBTile = P::kBTile;
+  constexpr int kSlots = P::kSlots;
+  constexpr int kCols = BN / 2;  // columns per epilogue thread
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = tc::align1024_shared(smem_raw);
-  __shared__ __align__(8) uint64_t full_bar[kOzStages], empty_bar[kOzStages];
+  __shared__ __align__(8) uint64_t full_bar[kSlots], empty_bar[kSlots];
   __shared__ __align__(8) uint64_t acc_full, acc_empty;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nk = (kdim + kOzBK - 1) / kOzBK;
-  const int chunks = (nk + chunk_kb - 1) / chunk_kb;
   const int total_tiles = m_tiles * n_tiles;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kOzStages; ++s) {
+    for (int s = 0; s < kSlots; ++s) {
       tc::mbar_init(&full_bar[s], 1);
       tc::mbar_init(&empty_bar[s], 1);
     }
@@ -285,74 +432,114 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
 
   if (warp == 0) {
     if (lane == 0) {
-      int it = 0;
-      for (int tile = blockIdx.x; tile < total_tiles && !abort_flag; tile += gridDim.x) {
+      int it = 0;  // slots filled
+      bool stop = false;
+      // Waits for the next slot and announces `bytes`; its barrier and address.
+      auto next_slot = [&](uint32_t bytes, uint64_t*& bar) -> uint8_t* {
+        const int slot = it % kSlots;
+        if ((it >= kSlots && !tc::mbar_wait(&empty_bar[slot], ((it / kSlots) - 1) & 1, limit_ns))) {
+          atomicOr(status, kStatusTimeout);
+          atomicExch(&abort_flag, 1);
+          return nullptr;
+        }
+        if (*(volatile int*)&abort_flag) return nullptr;
+        bar = &full_bar[slot];
+        if (bytes) tc::mbar_expect_tx(bar, bytes);
+        else tc::mbar_arrive(bar);
+        ++it;
+        return smem + P::offset(slot);
+      };
+      for (int tile = blockIdx.x; tile < total_tiles && !stop; tile += gridDim.x) {
         int mt, nt;
         oz_tile_coords(tile, m_tiles, n_tiles, mt, nt);
-        for (int kb = 0; kb < nk; ++kb, ++it) {
-          const int s = it % kOzStages;
-          if (it >= kOzStages && !tc::mbar_wait(&empty_bar[s], ((it / kOzStages) - 1) & 1, limit_ns)) {
-            atomicOr(status, kStatusTimeout);
-            atomicExch(&abort_flag, 1);
-            break;
+        const int m0 = mt * kOzBM, n0 = nt * BN;
+        for (int c0 = 0; c0 < nk && !stop; c0 += chunk_kb) {
+          const int c1 = min(nk, c0 + chunk_kb);
+          uint64_t* bar;
+          uint8_t* st;
+          for (int kb = c0; kb < c1 && !stop; ++kb) {
+            if (!(st = next_slot(P::kHigh, bar))) { stop = true; break; }
+            tc::tma_load_3d(st, &maps.a[1], bar, kb * kOzBK, m0, 3);
+            tc::tma_load_3d(st + 4 * kATile, &maps.b[1], bar, kb * kOzBK, n0, 0);
+            if (!(st = next_slot(P::kLow, bar))) { stop = true; break; }
+            tc::tma_load_3d(st, &maps.a[0], bar, kb * kOzBK, m0, 0);
+            tc::tma_load_3d(st + 3 * kATile, &maps.b[0], bar, kb * kOzBK, n0, 4);
           }
-          if (*(volatile int*)&abort_flag) break;
-          uint8_t* st = smem + (size_t)s * kStageBytes;
-          tc::mbar_expect_tx(&full_bar[s], kStageBytes);
-          for (int p = 0; p < S; ++p) {
-            tc::tma_load_2d(st + p * kATile, &maps.a[p], &full_bar[s], kb * kOzBK, mt * kOzBM);
-            tc::tma_load_2d(st + S * kATile + p * kBTile, &maps.b[p], &full_bar[s], kb * kOzBK, nt * kOzBN);
+          if (P::kPasses == 2) {
+            for (int kb = c0; kb < c1 && !stop; ++kb) {
+              if (!(st = next_slot(P::kLow, bar))) { stop = true; break; }
+              tc::tma_load_3d(st, &maps.a[0], bar, kb * kOzBK, m0, 0);
+              tc::tma_load_3d(st + 3 * kATile, &maps.b[0], bar, kb * kOzBK, n0, 0);
+            }
+            // an odd number of slabs leaves a low slot before the next high one
+            if (((c1 - c0) & 1) && !stop && !next_slot(0, bar)) stop = true;
           }
         }
       }
-      for (int j = (it > kOzStages ? it - kOzStages : 0); j < it; ++j)
-        tc::mbar_wait(&full_bar[j % kOzStages], (j / kOzStages) & 1, limit_ns);
+      // every issued load lands before the CTA may exit (own 1 s bound)
+      for (int j = (it > kSlots ? it - kSlots : 0); j < it; ++j)
+        tc::mbar_wait(&full_bar[j % kSlots], (j / kSlots) & 1, 1000000000ull);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int it = 0, gc = 0;
-      bool stop = false;
-      for (int tile = blockIdx.x; tile < total_tiles && !stop; tile += gridDim.x) {
-        for (int c = 0; c < chunks && !stop; ++c, ++gc) {
-          // the epilogue must have drained the previous chunk
-          if (gc >= 1 && !tc::mbar_wait(&acc_empty, (gc - 1) & 1, limit_ns)) {
-            atomicOr(status, kStatusTimeout);
-            atomicExch(&abort_flag, 1);
-            stop = true;
-            break;
+    // ---- MMA issuer: the warp stays converged, one lane issues ----
+    const bool lead = tc::elect_one();
+    int it = 0, gc = 0;
+    bool stop = false;
+    const uint64_t ring = tc::desc_k_sw64(tc::smem_u32(smem));
+    const uint32_t ring_lo = (uint32_t)ring, hi = (uint32_t)(ring >> 32);
+    auto wait_all = [&](uint64_t* bar, uint32_t parity) {
+      if (__all_sync(0xffffffffu, tc::mbar_wait(bar, parity, limit_ns))) return true;
+      if (lead) {
+        atomicOr(status, kStatusTimeout);
+        atomicExch(&abort_flag, 1);
+      }
+      stop = true;
+      return false;
+    };
+    auto take_slot = [&](int& slot) {
+      slot = it % kSlots;
+      const bool ok = wait_all(&full_bar[slot], (it / kSlots) & 1);
+      tc::tc_fence_after();
+      ++it;
+      return ok;
+    };
+    auto at = [&](int slot) { return ring_lo + (P::offset(slot) >> 4); };
+    for (int tile = blockIdx.x; tile < total_tiles && !stop; tile += gridDim.x) {
+      for (int c0 = 0; c0 < nk && !stop; c0 += chunk_kb) {
+        const int c1 = min(nk, c0 + chunk_kb);
+        // the epilogue must have drained the previous pass
+        if (gc >= 1 && !wait_all(&acc_empty, (gc - 1) & 1)) break;
+        tc::tc_fence_after();
+        for (int kb = c0; kb < c1; ++kb) {
+          int high, low;
+          if (!take_slot(high)) break;
+          const uint32_t ha = at(high), hb = ha + (4 * kATile >> 4);
+          if (lead) oz_issue<BN, kOzHighHigh>(ha, hb, hi, tmem, kb == c0);
+          if (!take_slot(low)) break;
+          const uint32_t la = at(low), lb = la + (3 * kATile >> 4);
+          if (lead) {
+            oz_issue<BN, kOzLowHigh>(la, hb, hi, tmem, kb == c0);
+            tc::mma_commit(&empty_bar[high]);
+            oz_issue<BN, kOzLowLow>(la, lb, hi, tmem, kb == c0);
+            tc::mma_commit(&empty_bar[low]);
           }
+        }
+        if (lead) tc::mma_commit(&acc_full);
+        ++gc;
+        if (P::kPasses == 2 && !stop) {
+          if (!wait_all(&acc_empty, (gc - 1) & 1)) break;
           tc::tc_fence_after();
-          const int kb0 = c * chunk_kb, kb1 = min(nk, kb0 + chunk_kb);
-          for (int kb = kb0; kb < kb1; ++kb, ++it) {
-            const int s = it % kOzStages;
-            if (!tc::mbar_wait(&full_bar[s], (it / kOzStages) & 1, limit_ns)) {
-              atomicOr(status, kStatusTimeout);
-              atomicExch(&abort_flag, 1);
-              stop = true;
-              break;
+          int slot;
+          for (int kb = c0; kb < c1; ++kb) {
+            if (!take_slot(slot)) break;
+            if (lead) {
+              oz_issue<BN, kOzSecondPass>(at(slot), at(slot) + (3 * kATile >> 4), hi, tmem, kb == c0);
+              tc::mma_commit(&empty_bar[slot]);
             }
-            tc::tc_fence_after();
-            const uint32_t sa = tc::smem_u32(smem + (size_t)s * kStageBytes);
-            const uint32_t sb = sa + S * kATile;
-#pragma unroll
-            for (int kk = 0; kk < kOzBK / 32; ++kk) {
-#pragma unroll
-              for (int d = 2; d <= S + 1; ++d) {
-                const uint32_t acc = tmem + (d - 2) * kOzBN;
-#pragma unroll
-                for (int p = 1; p <= S; ++p) {
-                  const int q = d - p;
-                  if (q < 1 || q > S) continue;
-                  const uint64_t ad = tc::desc_k_sw64(sa + (p - 1) * kATile + kk * 32);
-                  const uint64_t bd = tc::desc_k_sw64(sb + (q - 1) * kBTile + kk * 32);
-                  const bool first = (kb == kb0) && kk == 0 && p == max(1, d - S);
-                  tc::mma_i8(acc, ad, bd, kIdesc, first ? 0u : 1u);
-                }
-              }
-            }
-            tc::mma_commit(&empty_bar[s]);
           }
-          tc::mma_commit(&acc_full);
+          if (((c1 - c0) & 1) && !stop && take_slot(slot) && lead) tc::mma_commit(&empty_bar[slot]);
+          if (lead) tc::mma_commit(&acc_full);
+          ++gc;
         }
       }
     }
@@ -371,31 +558,42 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
       double sum[kCols];
 #pragma unroll
       for (int j = 0; j < kCols; ++j) sum[j] = 0.0;
-      for (int c = 0; c < chunks; ++c, ++gc) {
-        if (!tc::mbar_wait(&acc_full, gc & 1, limit_ns)) {
-          atomicOr(status, kStatusTimeout);
-          stop = true;
-          break;
-        }
-        tc::tc_fence_after();
-#pragma unroll 1
-        for (int d = 2; d <= S + 1; ++d) {
-          uint32_t r[32];
-          tc::tmem_ld32(tmem + (d - 2) * kOzBN + half * kCols + lane_base, r);
-          tc::tmem_wait_ld();
-          const double sc = ldexp(1.0, -7 * d);
+      // C into L2 while the products run (a warp's 32 rows are two or four lines a column)
+      if (!beta0) {
+        const int prow = mt * kOzBM + quad * 32 + lane, width = ep.complex_out ? 2 : 1;
+        const int pcol = (nt * BN + half * kCols) / width, pcols = kCols / width;
+        if (prow < ep.m && (lane & (16 / width - 1)) == 0)
+          for (int j = 0; j < pcols && pcol + j < ep.n; ++j)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(ep.C + ((size_t)prow + (size_t)(pcol + j) * ep.ldc) * width));
+      }
+      for (int c0 = 0; c0 < nk && !stop; c0 += chunk_kb) {
 #pragma unroll
-          for (int j = 0; j < kCols; ++j) sum[j] = fma((double)(int)r[j], sc, sum[j]);
+        for (int pass = 0; pass < P::kPasses; ++pass, ++gc) {
+          if (stop || !tc::mbar_wait(&acc_full, gc & 1, limit_ns)) {
+            atomicOr(status, kStatusTimeout);
+            stop = true;
+            break;
+          }
+          tc::tc_fence_after();
+          const uint32_t acc = tmem + half * kCols + lane_base;
+          if (BN == 64) {
+            oz_drain<5, 8, BN>(acc + 3 * BN, sum);
+            oz_drain<2, 4, BN>(acc, sum);
+          } else if (pass == 0) {
+            oz_drain<5, 8, BN>(acc, sum);
+          } else {
+            oz_drain<2, 4, BN>(acc, sum);
+          }
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&acc_empty);
         }
-        tc::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&acc_empty);
       }
       if (stop || *(volatile int*)&abort_flag) break;
       const int row = mt * kOzBM + quad * 32 + lane;
       if (row >= ep.m) continue;
       const int ei = max(ep.ea[row], -4000);  // all-zero rows keep the INT_MIN-like fill
-      const int col0 = nt * kOzBN + half * kCols;
+      const int col0 = nt * BN + half * kCols;
       // All C loads (and column exponents) of the tile row before any store:
       // a store followed by a load the compiler cannot prove disjoint would
       // cost a memory round trip per column.
@@ -457,44 +655,56 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
   if (warp == 1) tc::tmem_dealloc(tmem, 512);
 }
 
-template <int S>
-size_t oz_smem_bytes() {
-  return (size_t)kOzStages * S * (kOzBM * kOzBK + kOzBN * kOzBK) + 1024;
-}
-
-// K slabs per exact INT32 chunk: (products on the fullest diagonal) * 127^2 * k < 2^31.
+// K slabs per exact chunk: (products on the fullest diagonal) * 127^2 * k < 2^30, so
+// that a diagonal fits INT32 and four of them, 2^7 apart, stay below 2^51.
 template <int S>
 int oz_chunk_slabs() {
-  const long long kmax = (long long)INT32_MAX / (127LL * 127LL * S);
+  const long long kmax = (long long)(1 << 30) / (127LL * 127LL * S);
   return (int)(kmax / kOzBK);
+}
+
+template <int S, int BN>
+coral_status_t launch_ozaki(Handle* h, const OzMaps& maps, int mr, int nr, int kd, const OzEpi& ep) {
+  const size_t smem = 2 * ((size_t)OzPlan<BN>::kHigh + OzPlan<BN>::kLow) + 1024;
+  static uint64_t attr_devices = 0;  // bit d: attribute set on device d
+  const uint64_t bit = h->device < 64 ? (1ull << h->device) : 0;
+  if (!(attr_devices & bit) || !bit) {
+    CORAL_CUDA(h, cudaFuncSetAttribute(k_gemm_ozaki<S, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_devices |= bit;
+  }
+  const int m_tiles = (mr + kOzBM - 1) / kOzBM, n_tiles = (nr + BN - 1) / BN;
+  const int tiles = m_tiles * n_tiles;
+  const int grid = tiles < h->sm_count ? tiles : h->sm_count;
+  timed_begin(h);
+  k_gemm_ozaki<S, BN><<<grid, kOzThreads, smem, h->stream>>>(maps, kd, m_tiles, n_tiles, oz_chunk_slabs<S>(), ep,
+                                                             &h->words->status, h->wait_limit * 32ull);
+  coral_status_t s = launch_status(h);
+  timed_end(h);
+  return s;
 }
 
 template <int S>
 coral_status_t run_ozaki_gemm(Handle* h, const int8_t* ap, size_t a_piece, int mr, const int8_t* bp,
                               size_t b_piece, int nr, int kd, size_t kp, const OzEpi& ep) {
+  // Waves of tiles times a tile's cycles.  Both sides measured (us, 64 / 128 wide):
+  // 4096^3 1321 / 1175, 2048^3 198 / 185, 1000^3 42 / 73, 4096 x 512 x 64 25 / 32.
+  const long long slabs = (kd + kOzBK - 1) / kOzBK;
+  auto cost = [&](int bn, int slab_cycles, int tile_cycles) {
+    const long long tiles = (long long)((mr + kOzBM - 1) / kOzBM) * ((nr + bn - 1) / bn);
+    return (tiles + h->sm_count - 1) / h->sm_count * (slabs * slab_cycles + tile_cycles);
+  };
+  const int bn = cost(128, OzPlan<128>::kSlabCycles, OzPlan<128>::kTileCycles) <=
+                         cost(64, OzPlan<64>::kSlabCycles, OzPlan<64>::kTileCycles)
+                     ? 128
+                     : 64;
   OzMaps maps;
   std::memset(&maps, 0, sizeof(maps));
-  for (int p = 0; p < S; ++p) {
-    if (!encode_kmajor_map(&maps.a[p], ap + p * a_piece, 1, (uint64_t)kd, (uint64_t)mr, kp, kOzBK, kOzBM, 64) ||
-        !encode_kmajor_map(&maps.b[p], bp + p * b_piece, 1, (uint64_t)kd, (uint64_t)nr, kp, kOzBK, kOzBN, 64))
+  for (int i = 0; i < 2; ++i) {
+    if (!encode_slices_map(&maps.a[i], ap, kd, mr, S, kp, a_piece, kOzBK, kOzBM, 3 + i) ||
+        !encode_slices_map(&maps.b[i], bp, kd, nr, S, kp, b_piece, kOzBK, bn, 3 + i))
       return CORAL_ERR_NOT_SUPPORTED;
   }
-  const size_t smem = oz_smem_bytes<S>();
-  static uint64_t attr_devices = 0;  // bit d: attribute set on device d
-  const uint64_t bit = h->device < 64 ? (1ull << h->device) : 0;
-  if (!(attr_devices & bit) || !bit) {
-    CORAL_CUDA(h, cudaFuncSetAttribute(k_gemm_ozaki<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_devices |= bit;
-  }
-  const int m_tiles = (mr + kOzBM - 1) / kOzBM, n_tiles = (nr + kOzBN - 1) / kOzBN;
-  const int tiles = m_tiles * n_tiles;
-  const int grid = tiles < h->sm_count ? tiles : h->sm_count;
-  timed_begin(h);
-  k_gemm_ozaki<S><<<grid, kOzThreads, smem, h->stream>>>(maps, kd, m_tiles, n_tiles, oz_chunk_slabs<S>(),
-                                                         ep, &h->words->status, h->wait_limit * 32ull);
-  coral_status_t s = launch_status(h);
-  timed_end(h);
-  return s;
+  return bn == 128 ? launch_ozaki<S, 128>(h, maps, mr, nr, kd, ep) : launch_ozaki<S, 64>(h, maps, mr, nr, kd, ep);
 }
 
 constexpr int kOzSlices = 7;
@@ -528,8 +738,8 @@ coral_status_t dgemm_ozaki_core(Handle* h, char* sc, int op_a, int op_b, size_t 
   coral_status_t s = launch_row_exponent(h, A, lda, (int)m, (int)k, a_km, ea);
   if (s != CORAL_OK) return s;
   if ((s = launch_row_exponent(h, B, ldb, (int)n, (int)k, b_km, eb)) != CORAL_OK) return s;
-  dim3 gsa((unsigned)((kp + 31) / 32), (unsigned)((m + 31) / 32));
-  dim3 gsb((unsigned)((kp + 31) / 32), (unsigned)((n + 31) / 32));
+  dim3 gsa((unsigned)((kp + 127) / 128), (unsigned)((m + 31) / 32));
+  dim3 gsb((unsigned)((kp + 127) / 128), (unsigned)((n + 31) / 32));
   if (a_km) k_slice_real<S, true><<<gsa, 256, 0, h->stream>>>(A, lda, (int)m, (int)k, ea, ap, kp, a_piece);
   else k_slice_real<S, false><<<gsa, 256, 0, h->stream>>>(A, lda, (int)m, (int)k, ea, ap, kp, a_piece);
   if ((s = launch_status(h)) != CORAL_OK) return s;

@@ -83,6 +83,16 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// 3-D tiled TMA load into this CTA's shared memory, completing on `bar`.
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar,
+                                            int32_t c0, int32_t c1, int32_t c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+
 // Makes this thread's generic-proxy shared-memory writes visible to the async
 // proxy (tcgen05.mma operand reads); issue before arriving on the barrier the
 // MMA issuer waits on.
@@ -92,6 +102,20 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
+// True in one lane of a converged warp.  An MMA issuer that runs its loop with
+// the whole warp and only issues under this test keeps descriptors in uniform
+// registers: 25 cycles per instruction against 45 when one lane runs the loop
+// (measured, kind::i8), which bounds products of 64 columns or fewer.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b32 r;\n\t"
+      "elect.sync r|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
 }
 
 // ---- TMEM ------------------------------------------------------------------
@@ -161,15 +185,26 @@ __device__ __forceinline__ void mma_f16_ca(uint32_t tmem_d, uint64_t adesc, uint
   }
 }
 
-// D[tmem] (+)= A * B^T, kind::i8 (signed 8-bit operands, s32 accumulate).
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                       uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// D[tmem] (+)= A * B^T, kind::i8 (signed 8-bit operands, s32 accumulate), with
+// the A operand kept in the collector buffer as for mma_f16_ca.  The
+// descriptors come as their low words and one common high word: inside the
+// ring they differ by a number of 16-byte units, one addition per operand.
+template <int kCollect>
+__device__ __forceinline__ void mma_i8_ca(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
+                                          uint32_t idesc, uint32_t accumulate) {
+#define CORAL_MMA_I8(usage)                                                                          \
+  asm volatile(                                                                                      \
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"                                                    \
+      "setp.ne.b32 p, %5, 0;\n\t"                                                                    \
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"                                             \
+      "tcgen05.mma.cta_group::1.kind::i8" usage " [%0], a, b, %4, p;\n\t}\n" ::"r"(tmem_d),          \
+      "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)                                     \
+      : "memory")
+  if constexpr (kCollect == kCollectFill) CORAL_MMA_I8(".collector::a::fill");
+  else if constexpr (kCollect == kCollectUse) CORAL_MMA_I8(".collector::a::use");
+  else if constexpr (kCollect == kCollectLastUse) CORAL_MMA_I8(".collector::a::lastuse");
+  else CORAL_MMA_I8("");
+#undef CORAL_MMA_I8
 }
 
 // Arrives on `bar` once every previously issued tcgen05.mma of this thread completed.
@@ -298,6 +333,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
+// 32 lanes x 8 consecutive 32-bit columns.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -352,5 +393,10 @@ __host__ __device__ constexpr uint32_t idesc_s8_s32(int M, int N) {
 bool encode_kmajor_map(CUtensorMap* map, const void* base, int elem_bytes, uint64_t inner,
                        uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner,
                        uint32_t box_outer, int swizzle_bytes = 128);
+// Same for byte slices [slices][rows][inner], 64-byte swizzle: a box of box_slices
+// x box_rows x box_inner bytes.
+bool encode_slices_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t slices,
+                       uint64_t row_stride, uint64_t slice_stride, uint32_t box_inner, uint32_t box_rows,
+                       uint32_t box_slices);
 
 }  // namespace coral
