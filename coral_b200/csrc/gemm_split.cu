@@ -9,7 +9,7 @@
 //
 // Pipeline per call:
 //   1. split pre-pass: op(A) -> pieces [m][kp] and op(B)^T -> pieces [n][kp],
-//      bf16, K contiguous (kp = k rounded up to 8 so rows are 16-byte
+//      bf16, K contiguous (rows of kp, see piece_pitch: 16-byte
 //      multiples).  Transposes through shared memory when the stored matrix
 //      is contiguous along M/N.  Complex operands use the 4M mapping folded
 //      into one real GEMM: A'' = [Re A | Im A] (k' = 2k) and rows
@@ -446,6 +446,75 @@ struct EpiParams {
   int complex_out;   // 1: accumulator columns (2j, 2j+1) are (Re, Im) of C column j
 };
 
+constexpr int kCGroup = 8;  // C columns loaded together by the epilogue
+
+// Writes a thread's row of a tile: kCols accumulator columns from col0 (complex:
+// pairs of them are Re and Im of a column of C).  C is read in groups of kCGroup
+// columns, the next group's loads ahead of this group's stores: a store followed
+// by a load the compiler cannot prove disjoint would otherwise cost a memory
+// round trip per column.  Pointers advance by a column and beta == 0 takes the
+// same multiply-add with -0 for C (exact: beta * -0 + v = v), because the code
+// runs once per tile, unrolled over the accumulators, and much of what it costs is
+// fetching it (4096 x 4096 x 256: 64 -> 51 us against an address and three
+// selections per element; groups of 16 columns spill, 66).
+template <int kCols>
+__device__ __forceinline__ void store_row(const EpiParams& ep, int row, int col0, const float (&sum)[kCols]) {
+  const bool read_c = !(ep.beta_re == 0.f && ep.beta_im == 0.f);
+  if (!ep.complex_out) {
+    constexpr int G = kCGroup;
+    float* to = ep.C + row + (size_t)col0 * ep.ldc;
+    const float* from = to;
+    const int cols = ep.n - col0;
+    float cv[G];
+    auto load = [&](int g) {
+#pragma unroll
+      for (int j = 0; j < G; ++j, from += ep.ldc) {
+        cv[j] = -0.f;
+        if (read_c && g + j < cols) cv[j] = *from;
+      }
+    };
+    load(0);
+#pragma unroll
+    for (int g = 0; g < kCols; g += G) {
+      float out[G];
+#pragma unroll
+      for (int j = 0; j < G; ++j) out[j] = fmaf(ep.beta_re, cv[j], ep.alpha_re * sum[g + j]);
+      if (g + G < kCols) load(g + G);
+#pragma unroll
+      for (int j = 0; j < G; ++j, to += ep.ldc)
+        if (g + j < cols) *to = out[j];
+    }
+  } else {
+    const bool beta1 = ep.beta_re == 1.f && ep.beta_im == 0.f;
+    float2* crow = reinterpret_cast<float2*>(ep.C) + row;
+#pragma unroll
+    for (int g = 0; g < kCols / 2; g += kCGroup / 2) {
+      float2 cvs[kCGroup / 2];
+#pragma unroll
+      for (int j = 0; j < kCGroup / 2; ++j)
+        cvs[j] = (read_c && col0 / 2 + g + j < ep.n) ? crow[(size_t)(col0 / 2 + g + j) * ep.ldc]
+                                                     : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < kCGroup / 2; ++j) {
+        const int col = col0 / 2 + g + j;
+        if (col < ep.n) {
+          const float ar = sum[2 * (g + j)], ai = sum[2 * (g + j) + 1];
+          float2 v = make_float2(ep.alpha_re * ar - ep.alpha_im * ai, ep.alpha_re * ai + ep.alpha_im * ar);
+          if (read_c) {
+            const float2 cv = cvs[j];
+            if (beta1) { v.x += cv.x; v.y += cv.y; }
+            else {
+              v.x += ep.beta_re * cv.x - ep.beta_im * cv.y;
+              v.y += ep.beta_re * cv.y + ep.beta_im * cv.x;
+            }
+          }
+          crow[(size_t)col * ep.ldc] = v;
+        }
+      }
+    }
+  }
+}
+
 // Tile order: groups of 16 M-tiles sweep all N-tiles, so CTAs resident at
 // the same time share A and B slabs through L2.
 __device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, int& mt, int& nt) {
@@ -472,7 +541,6 @@ __device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, 
 // partial sum goes through; the register adds round to nearest.
 constexpr int kEpiWarps = 8;
 constexpr int kSplitThreads = 64 + 32 * kEpiWarps;
-constexpr int kCGroup = 8;  // C columns loaded together by the epilogue
 
 template <int NP, int BN>
 __global__ void __launch_bounds__(kSplitThreads, 1)
@@ -617,8 +685,6 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
     const int quad = warp & 3;           // TMEM lane quadrant this warp may access
     const int half = ew >> 2;            // column half of the tile
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-    const bool beta0 = ep.beta_re == 0.f && ep.beta_im == 0.f;
-    const bool beta1 = ep.beta_re == 1.f && ep.beta_im == 0.f;
     int gc = 0;
     bool stop = false;
     for (int item = blockIdx.x; item < total_items && !stop; item += gridDim.x) {
@@ -659,53 +725,8 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
 #pragma unroll
         for (int j = 0; j < kCols; ++j)
           if (col0 + j < ws_cols) wp[(size_t)(col0 + j) * ep.m] = sum[j];
-      } else if (!ep.complex_out) {
-        // C is read in groups of kCGroup columns, all loads of a group before
-        // any store: a store followed by a load the compiler cannot prove
-        // disjoint would otherwise cost a memory round trip per column.
-        float* crow = ep.C + row;
-#pragma unroll
-        for (int g = 0; g < kCols; g += kCGroup) {
-          float cv[kCGroup];
-#pragma unroll
-          for (int j = 0; j < kCGroup; ++j)
-            cv[j] = (!beta0 && col0 + g + j < ep.n) ? crow[(size_t)(col0 + g + j) * ep.ldc] : 0.f;
-#pragma unroll
-          for (int j = 0; j < kCGroup; ++j) {
-            const int col = col0 + g + j;
-            if (col < ep.n) {
-              const float v = ep.alpha_re * sum[g + j];
-              crow[(size_t)col * ep.ldc] = beta0 ? v : beta1 ? cv[j] + v : ep.beta_re * cv[j] + v;
-            }
-          }
-        }
       } else {
-        float2* crow = reinterpret_cast<float2*>(ep.C) + row;
-#pragma unroll
-        for (int g = 0; g < kCols / 2; g += kCGroup / 2) {
-          float2 cvs[kCGroup / 2];
-#pragma unroll
-          for (int j = 0; j < kCGroup / 2; ++j)
-            cvs[j] = (!beta0 && col0 / 2 + g + j < ep.n) ? crow[(size_t)(col0 / 2 + g + j) * ep.ldc]
-                                                          : make_float2(0.f, 0.f);
-#pragma unroll
-          for (int j = 0; j < kCGroup / 2; ++j) {
-            const int col = col0 / 2 + g + j;
-            if (col < ep.n) {
-              const float ar = sum[2 * (g + j)], ai = sum[2 * (g + j) + 1];
-              float2 v = make_float2(ep.alpha_re * ar - ep.alpha_im * ai, ep.alpha_re * ai + ep.alpha_im * ar);
-              if (!beta0) {
-                const float2 cv = cvs[j];
-                if (beta1) { v.x += cv.x; v.y += cv.y; }
-                else {
-                  v.x += ep.beta_re * cv.x - ep.beta_im * cv.y;
-                  v.y += ep.beta_re * cv.y + ep.beta_im * cv.x;
-                }
-              }
-              crow[(size_t)col * ep.ldc] = v;
-            }
-          }
-        }
+        store_row<kCols>(ep, row, col0, sum);
       }
     }
   }
@@ -913,8 +934,6 @@ k_gemm_split_pair(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles,
     const int quad = warp & 3;
     const int half = ew >> 2;
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-    const bool beta0 = ep.beta_re == 0.f && ep.beta_im == 0.f;
-    const bool beta1 = ep.beta_re == 1.f && ep.beta_im == 0.f;
     int gc = 0;
     bool stop = false;
     for (int item = cluster; item < total_items && !stop; item += nclusters) {
@@ -955,50 +974,8 @@ k_gemm_split_pair(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles,
 #pragma unroll
         for (int j = 0; j < kCols; ++j)
           if (col0 + j < ws_cols) wp[(size_t)(col0 + j) * ep.m] = sum[j];
-      } else if (!ep.complex_out) {
-        float* crow = ep.C + row;
-#pragma unroll
-        for (int g = 0; g < kCols; g += kCGroup) {
-          float cv[kCGroup];
-#pragma unroll
-          for (int j = 0; j < kCGroup; ++j)
-            cv[j] = (!beta0 && col0 + g + j < ep.n) ? crow[(size_t)(col0 + g + j) * ep.ldc] : 0.f;
-#pragma unroll
-          for (int j = 0; j < kCGroup; ++j) {
-            const int col = col0 + g + j;
-            if (col < ep.n) {
-              const float v = ep.alpha_re * sum[g + j];
-              crow[(size_t)col * ep.ldc] = beta0 ? v : beta1 ? cv[j] + v : ep.beta_re * cv[j] + v;
-            }
-          }
-        }
       } else {
-        float2* crow = reinterpret_cast<float2*>(ep.C) + row;
-#pragma unroll
-        for (int g = 0; g < kCols / 2; g += kCGroup / 2) {
-          float2 cvs[kCGroup / 2];
-#pragma unroll
-          for (int j = 0; j < kCGroup / 2; ++j)
-            cvs[j] = (!beta0 && col0 / 2 + g + j < ep.n) ? crow[(size_t)(col0 / 2 + g + j) * ep.ldc]
-                                                          : make_float2(0.f, 0.f);
-#pragma unroll
-          for (int j = 0; j < kCGroup / 2; ++j) {
-            const int col = col0 / 2 + g + j;
-            if (col < ep.n) {
-              const float ar = sum[2 * (g + j)], ai = sum[2 * (g + j) + 1];
-              float2 v = make_float2(ep.alpha_re * ar - ep.alpha_im * ai, ep.alpha_re * ai + ep.alpha_im * ar);
-              if (!beta0) {
-                const float2 cv = cvs[j];
-                if (beta1) { v.x += cv.x; v.y += cv.y; }
-                else {
-                  v.x += ep.beta_re * cv.x - ep.beta_im * cv.y;
-                  v.y += ep.beta_re * cv.y + ep.beta_im * cv.x;
-                }
-              }
-              crow[(size_t)col * ep.ldc] = v;
-            }
-          }
-        }
+        store_row<kCols>(ep, row, col0, sum);
       }
     }
   }
@@ -1180,8 +1157,8 @@ coral_status_t run_split_gemm_pair(Handle* h, const __nv_bfloat16* ap, size_t a_
 
 // Tile width and split-K factor for a split-BF16 GEMM of op(A) (mr x kd)
 // times B-rows (nr x kd): the handle's explicit choice, else its selector,
-// else the default rule (full-width tiles; split K when the output tiles
-// cannot fill the GPU and K is deep).
+// else the default rule (256 columns, or 128 where those fill one wave at most or
+// K is short; K in parts when the output tiles cannot fill the GPU and K is deep).
 SplitConfig choose_split_config(Handle* h, const SplitShape& sh) {
   const int products = sh.products, mr = sh.mr, nr = sh.nr, kd = sh.kd;
   SplitConfig c{products == 3 ? 256 : 128, 1};
@@ -1196,20 +1173,27 @@ SplitConfig choose_split_config(Handle* h, const SplitShape& sh) {
   } else if (h->selector && select_split_config(h, sh, &c)) {
     // selector decided
   } else {
-    const int tiles = ((mr + kBM - 1) / kBM) * ((nr + c.bn - 1) / c.bn);
+    const int m_tiles = (mr + kBM - 1) / kBM;
+    const int tiles = m_tiles * ((nr + c.bn - 1) / c.bn), tiles128 = m_tiles * ((nr + 127) / 128);
     const int pair_tiles = ((mr + kPairTile - 1) / kPairTile) * ((nr + kPairTile - 1) / kPairTile);
-    if (pair_tiles >= h->sm_count) {
-      // At least two waves of 256 x 256 tiles over the resident CTA pairs:
-      // the pair tiles read half as much of B per flop from shared memory.
-      c.pair = 1;
-      c.bn = 256;
-    } else if (tiles * 2 <= h->sm_count && nk >= 16) {
+    if (tiles * 2 <= h->sm_count && nk >= 16) {
+      // split K (its parts also bound how many tensor-core additions a sum goes through)
       int sp = h->sm_count / tiles;
       sp = sp > 16 ? 16 : sp;
       sp = sp > nk ? nk : sp;
       int p2 = 1;  // largest power of two <= sp (the tuned candidate set)
       while (p2 * 2 <= sp) p2 *= 2;
       c.splits = p2;
+    } else if (tiles128 <= h->sm_count || (nk <= 5 && products == 3)) {
+      // One wave of 128 x 128 tiles, or a product whose time goes into C: half
+      // the columns per tile are drained and written in half the time (us, 128 /
+      // 256 wide: 700^3 19.5 / 24.7, 1500^3 34.9 / 41.5, 4096 x 4096 x 256 47 / 57).
+      c.bn = 128;
+    } else if (pair_tiles >= h->sm_count) {
+      // At least two waves of 256 x 256 tiles over the resident CTA pairs:
+      // the pair tiles read half as much of B per flop from shared memory.
+      c.pair = 1;
+      c.bn = 256;
     }
   }
   if (products == 6 && !c.pair) c.bn = 128;
@@ -1232,12 +1216,21 @@ coral_status_t dispatch_split_gemm(Handle* h, const __nv_bfloat16* ap, size_t a_
   return run_split_gemm<NP, 128>(h, ap, a_piece, mr, bp, b_piece, nr, kd, kp, c.splits, ws, ep);
 }
 
+// Row pitch of the pieces in bf16 elements: a multiple of 8 (TMA's 16-byte
+// strides), and of 64 where K is deep enough for that to cost little memory.  The
+// 64-byte row of a slab then lies in one 128-byte line; at other pitches it
+// straddles two for half of the rows, and the loads of 2001 x 3003 x 1027 bounded
+// the GEMM kernel (pitch 1032 against 1088: 80 -> 53 us; 3000^3 194 -> 119).
+size_t piece_pitch(size_t k) {
+  return k >= 512 ? (k + 63) & ~size_t(63) : (k + 7) & ~size_t(7);
+}
+
 template <int NP>
 coral_status_t sgemm_split_impl(Handle* h, int op_a, int op_b, size_t m, size_t n, size_t k,
                                 float alpha, const float* A, size_t lda, const float* B, size_t ldb,
                                 float beta, float* C, size_t ldc) {
   constexpr int NPC = SplitPlan<NP>::kPieces;
-  const size_t kp = (k + 7) & ~size_t(7);
+  const size_t kp = piece_pitch(k);
   const size_t a_piece = m * kp, b_piece = n * kp;
   const size_t a_bytes = (NPC * a_piece * 2 + 255) & ~size_t(255);
   const size_t b_bytes = (NPC * b_piece * 2 + 255) & ~size_t(255);
@@ -1270,7 +1263,7 @@ coral_status_t cgemm_split_3m(Handle* h, int op_a, int op_b, size_t m, size_t n,
                               float2 alpha, const float2* A, size_t lda, const float2* B, size_t ldb,
                               float2 beta, float2* C, size_t ldc) {
   constexpr int NPC = SplitPlan<NP>::kPieces;
-  const size_t kp = (k + 7) & ~size_t(7);
+  const size_t kp = piece_pitch(k);
   const size_t a_piece = m * kp, b_piece = n * kp;
   const size_t a_part = NPC * a_piece, b_part = NPC * b_piece;
   const size_t a_bytes = (3 * a_part * 2 + 255) & ~size_t(255);
@@ -1319,7 +1312,7 @@ coral_status_t cgemm_split_impl(Handle* h, int op_a, int op_b, size_t m, size_t 
     return cgemm_split_3m<NP>(h, op_a, op_b, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
   constexpr int NPC = SplitPlan<NP>::kPieces;
   const size_t k2 = 2 * k;
-  const size_t kp = (k2 + 7) & ~size_t(7);
+  const size_t kp = piece_pitch(k2);
   const size_t a_piece = m * kp, b_piece = 2 * n * kp;
   const size_t a_bytes = (NPC * a_piece * 2 + 255) & ~size_t(255);
   const size_t b_bytes = (NPC * b_piece * 2 + 255) & ~size_t(255);
@@ -1330,9 +1323,7 @@ coral_status_t cgemm_split_impl(Handle* h, int op_a, int op_b, size_t m, size_t 
   if (!sc) return CORAL_ERR_ALLOC;
   __nv_bfloat16* ap = reinterpret_cast<__nv_bfloat16*>(sc);
   __nv_bfloat16* bp = reinterpret_cast<__nv_bfloat16*>(sc + a_bytes);
-  if (kp != k2) {  // zero the row tails so every byte TMA may read is defined
-    CORAL_CUDA(h, cudaMemsetAsync(sc, 0, a_bytes + b_bytes, h->stream));
-  }
+  // (row tails past k2 stay undefined: the tensor maps end at k2 and fill zeros)
   dim3 ga((unsigned)((k + 31) / 32), (unsigned)((m + 31) / 32));
   const bool ca = op_a == CORAL_CONJ_TRANSPOSE, cbj = op_b == CORAL_CONJ_TRANSPOSE;
   if (op_a == CORAL_NO_TRANSPOSE)
