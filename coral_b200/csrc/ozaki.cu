@@ -709,10 +709,17 @@ coral_status_t run_ozaki_gemm(Handle* h, const int8_t* ap, size_t a_piece, int m
 
 constexpr int kOzSlices = 7;
 
+// Row pitch of the slices in bytes: a multiple of 16 (TMA's strides), and of 128
+// where K is deep enough for that to cost little memory, so that a slab's 64-byte
+// row never straddles two lines.
+size_t slice_pitch(size_t k) {
+  return k >= 1024 ? (k + 127) & ~size_t(127) : (k + 15) & ~size_t(15);
+}
+
 // Device bytes the real Ozaki GEMM needs for its slices and exponents.
 size_t dgemm_ozaki_bytes(size_t m, size_t n, size_t k) {
   constexpr int S = kOzSlices;
-  const size_t kp = (k + 15) & ~size_t(15);
+  const size_t kp = slice_pitch(k);
   const size_t a_bytes = (S * m * kp + 1023) & ~size_t(1023);
   const size_t b_bytes = (S * n * kp + 1023) & ~size_t(1023);
   const size_t e_bytes = ((m + n) * sizeof(int) + 255) & ~size_t(255);
@@ -725,7 +732,7 @@ coral_status_t dgemm_ozaki_core(Handle* h, char* sc, int op_a, int op_b, size_t 
                                 double alpha, const double* A, size_t lda, const double* B,
                                 size_t ldb, double beta, double* C, size_t ldc) {
   constexpr int S = kOzSlices;
-  const size_t kp = (k + 15) & ~size_t(15);
+  const size_t kp = slice_pitch(k);
   const size_t a_piece = m * kp, b_piece = n * kp;
   const size_t a_bytes = (S * a_piece + 1023) & ~size_t(1023);
   const size_t b_bytes = (S * b_piece + 1023) & ~size_t(1023);
@@ -865,7 +872,7 @@ coral_status_t zgemm_ozaki_impl(Handle* h, int op_a, int op_b, size_t m, size_t 
                                 size_t ldb, double2 beta, double2* C, size_t ldc) {
   constexpr int S = kOzSlices;
   const size_t k2 = 2 * k;
-  const size_t kp = (k2 + 15) & ~size_t(15);
+  const size_t kp = slice_pitch(k2);
   const size_t a_piece = m * kp, b_piece = 2 * n * kp;
   const size_t a_bytes = (S * a_piece + 1023) & ~size_t(1023);
   const size_t b_bytes = (S * b_piece + 1023) & ~size_t(1023);
@@ -887,7 +894,7 @@ coral_status_t zgemm_ozaki_impl(Handle* h, int op_a, int op_b, size_t m, size_t 
                                   cudaMemcpyDeviceToDevice, h->stream));
   CORAL_CUDA(h, cudaMemcpy2DAsync(eb2 + 1, 2 * sizeof(int), ebs, sizeof(int), sizeof(int), n,
                                   cudaMemcpyDeviceToDevice, h->stream));
-  if (kp != k2) CORAL_CUDA(h, cudaMemsetAsync(sc, 0, a_bytes + b_bytes, h->stream));
+  // (row tails past k2 stay undefined: the tensor maps end at k2 and fill zeros)
   const bool ca = op_a == CORAL_CONJ_TRANSPOSE, cbj = op_b == CORAL_CONJ_TRANSPOSE;
   const dim3 ga((unsigned)((k + 31) / 32), (unsigned)((m + 31) / 32));  // 32 x 32 slicing tiles
   const dim3 gb((unsigned)((k + 31) / 32), (unsigned)((n + 31) / 32));
