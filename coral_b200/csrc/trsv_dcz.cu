@@ -11,17 +11,26 @@
 //      masked, unit diagonal applied, conjugated for op C), forms the
 //      reciprocals of its diagonal and scales each row by its reciprocal
 //      (negated, ready for the updates), and reads its right-hand side;
-//   2. for every earlier block k in solve order: loads its panel tile of
-//      op(A) into registers, then reads x_k from block k's published slots
-//      and accumulates op(A)(b, k) x_k -- four threads per row, 16 columns
-//      each;
+//   2. for every earlier block k in solve order: holds its panel tile of
+//      op(A) in registers (loaded while block k - 1 was waited for), reads x_k
+//      from block k's published slots and accumulates op(A)(b, k) x_k -- four
+//      threads per row, 16 columns each;
 //   3. solves the row-scaled system by forward (backward) substitution in
 //      one warp, fully unrolled (the diagonal block is never inverted: FP64
-//      substitution as the reference does, dtrlsv.rs);
-//   4. writes x_b over b, pushes it into the shared memory of the later CTAs
-//      of its cluster (the next block's first) and publishes it in its slots
-//      for later clusters: within a cluster a block's solution reaches the
-//      next one through distributed shared memory instead of an L2 round trip.
+//      substitution as the reference does, dtrlsv.rs), and pushes the result
+//      from its registers into the shared memory of the next CTA;
+//   4. writes x_b over b, pushes it to the cluster's other later CTAs and
+//      publishes it in its slots for later clusters: within a cluster a block's
+//      solution reaches the next one through distributed shared memory instead
+//      of an L2 round trip.
+// Bound: the chain of n / 64 hops (the 67 MB of DTRSV's n = 4096 triangle would
+// stream in 10 us).  A hop's cycles in DTRSV, before and after this form: last
+// tile's products and reduction 1250 -> 630 (pairs of x_k by 16-byte loads that
+// neighbouring lanes share, on padded banks), substitution 2640 -> 1600 (see
+// substitute()), hand-over about 700.  n = 4096, op N: DTRSV 153 -> 105 us,
+// CTRSV 172 -> 124, ZTRSV 262 -> 184; n = 16384: 797 -> 610, 827 -> 645,
+// 1464 -> 1046; n = 64 (the reciprocals of the diagonal in one division per lane,
+// the loads all in flight): 8.6 -> 5.2, 9.6 -> 5.9, 10.5 -> 7.3.
 // Slots: every 32-bit word of a block's solution is published as one 64-bit
 // slot (epoch << 32) | word, so a single load delivers both the readiness of
 // that word and its value (aligned 64-bit accesses are single-copy atomic):
@@ -43,12 +52,12 @@ namespace {
 // 200 us, ctrsv 250 against 187 us), and a complex128 block of 128 rows
 // would not fit in shared memory.
 template <typename T> constexpr int kTBOf = 64;
-// Substitution form per element type (see substitute_strided() and
-// substitute()), as measured at n = 4096: two consecutive rows per lane for
-// double (dtrsv 173 us, against 200 strided); rows 32 apart for complex,
-// whose wider elements make the consecutive form slower (ctrsv 236 against
-// 187 us, ztrsv 356 against 277 us).
-template <typename T> constexpr int kRowsPerLaneOf = std::is_same<T, double>::value ? 2 : 0;   // 0: strided
+// Rows solved together (see substitute()).
+template <typename T> constexpr int kCornerOf = std::is_same<T, double>::value ? 8 : 4;
+// Row pitch of the diagonal block in shared memory: 16-byte aligned pairs of
+// columns, and lanes on consecutive rows on different banks.
+template <typename T> constexpr int kPitchOf = kTBOf<T> + (sizeof(T) == 16 ? 1 : 2);
+template <typename T> struct alignas(16) Two { T x, y; };
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long v;
@@ -79,69 +88,68 @@ constexpr int kDczClMax = 16;  // CTAs per cluster: 16, or 8 where 16 cannot be 
 // 32-bit words per element (slots per element).
 template <typename T> constexpr int kWords = (int)(sizeof(T) / 4);
 
-// Substitution on the row-scaled diagonal block in one warp, fully unrolled.
-// D holds -op(A)(i, j) / op(A)(i, i) off the diagonal and v the scaled
-// right-hand side, so every x_i is its row's final v_i.
-//
-// Strided form: lane owns rows lane + 32 m (m < TB / 32).  At step j the
-// owner's value is x_j; it is broadcast and every later row i takes
-// v_i += D[i][j] x_j -- one shuffle round per row on the critical path.
-template <typename T, int TB, bool kLower>
-__device__ __forceinline__ void substitute_strided(const T (*D)[TB + 1], T (&v)[TB / 32], int lane) {
+// Substitution on the row-scaled diagonal block in one warp, fully unrolled, by
+// corners of B rows.  D (in solve order) holds -op(A)(i, j) / op(A)(i, i) below
+// the diagonal and v the scaled right-hand side of rows lane + 32 h, so every
+// x_i is its row's final v_i.  The lanes that own the next B rows hand them to
+// all (xs, two halves in turn); every lane solves their B x B corner -- the same
+// products in every lane, but one multiply-add per row on the chain and no
+// exchange -- while it takes the products off its own later rows.  Cycles of the
+// 64 rows, one warp alone, double: 1540 (B = 8), 1800 (B = 4), 2290 by one
+// broadcast per row; a wider product makes the 28 of an 8 x 8 corner the bound,
+// so complex takes B = 4 (complex64 3260 -> 1950, complex128 4400 -> 3150).
+template <typename T, int TB, int B, int P>
+__device__ __forceinline__ void substitute(const T* D, T* xs, T (&v)[TB / 32], int lane) {
   using F = Fld<T>;
+  using T2 = Two<T>;
+  constexpr int H = TB / 32, C = 32 / B;
 #pragma unroll
-  for (int s = 0; s < TB; ++s) {
-    const int j = kLower ? s : TB - 1 - s;
-    const T xj = F::shfl(v[j / 32], j & 31);
+  for (int s = 0; s < TB / B; ++s) {
+    T2 co[B][B / 2], ro[H][B / 2];
 #pragma unroll
-    for (int m = 0; m < TB / 32; ++m) {
-      const int i = lane + 32 * m;
-      if (kLower ? i > j : i < j) F::mac(v[m], D[i][j], xj);
+    for (int j = 0; j < B / 2; ++j) {
+#pragma unroll
+      for (int i = 2 * j + 1; i < B; ++i)
+        co[i][j] = *reinterpret_cast<const T2*>(D + (B * s + i) * P + B * s + 2 * j);
     }
-  }
-}
-
-// Consecutive form: lane l < TB / R owns
-// the R consecutive rows R l .. R l + R - 1 (v[0..R-1]).  In solve order, the
-// owner of the next R rows finishes them among themselves (R - 1 dependent
-// multiply-adds, no communication), broadcasts the R values, and every lane
-// whose rows come later applies them.  The critical path per R rows is R
-// multiply-adds and one shuffle round, against one shuffle per row when each
-// lane owns rows 32 apart.
-template <typename T, int TB, int R, bool kLower>
-__device__ __forceinline__ void substitute(const T (*D)[TB + 1], T (&v)[R], int lane) {
-  using F = Fld<T>;
-  constexpr int P = TB / R;   // owner lanes
+    T* xb = xs + B * (s & 1);
+    if (lane / B == s % C) xb[lane % B] = v[s / C];
+    __syncwarp();
+    T q[B];
 #pragma unroll
-  for (int s = 0; s < P; ++s) {
-    const int p = kLower ? s : P - 1 - s;
-    const int j0 = p * R;
-    if (lane == p) {
-      if (kLower) {
-#pragma unroll
-        for (int a = 0; a < R; ++a)
-#pragma unroll
-          for (int b = a + 1; b < R; ++b) F::mac(v[b], D[j0 + b][j0 + a], v[a]);
-      } else {
-#pragma unroll
-        for (int a = R - 1; a >= 0; --a)
-#pragma unroll
-          for (int b = a - 1; b >= 0; --b) F::mac(v[b], D[j0 + b][j0 + a], v[a]);
-      }
+    for (int j = 0; j < B; j += 2) {
+      const T2 t = *reinterpret_cast<const T2*>(xb + j);
+      q[j] = t.x;
+      q[j + 1] = t.y;
     }
-    T xr[R];
 #pragma unroll
-    for (int a = 0; a < R; ++a) xr[a] = F::shfl(v[a], p);
-    if (lane < P && (kLower ? lane > p : lane < p)) {
-      const int i0 = lane * R;
-      // the next owner's first row to finish gets its updates first
+    for (int j = 0; j < B / 2; ++j)
 #pragma unroll
-      for (int bb = 0; bb < R; ++bb) {
-        const int b = kLower ? bb : R - 1 - bb;
+      for (int h = 0; h < H; ++h)
+        if (32 * (h + 1) > B * (s + 1))
+          ro[h][j] = *reinterpret_cast<const T2*>(D + (lane + 32 * h) * P + B * s + 2 * j);
+    T w[H];
 #pragma unroll
-        for (int a = 0; a < R; ++a) F::mac(v[b], D[i0 + b][j0 + a], xr[a]);
-      }
+    for (int h = 0; h < H; ++h) w[h] = v[h];
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+#pragma unroll
+      for (int i = j + 1; i < B; ++i) F::mac(q[i], j & 1 ? co[i][j / 2].y : co[i][j / 2].x, q[j]);
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+        if (32 * (h + 1) > B * (s + 1)) F::mac(w[h], j & 1 ? ro[h][j / 2].y : ro[h][j / 2].x, q[j]);
     }
+    T own[B];  // q[lane % B], by bits (indexing q would put it in local memory)
+#pragma unroll
+    for (int j = 0; j < B; ++j) own[j] = q[j];
+#pragma unroll
+    for (int m = B / 2; m > 0; m /= 2)
+#pragma unroll
+      for (int j = 0; j < m; ++j) own[j] = lane & m ? own[j + m] : own[j];
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+      if (lane + 32 * h >= B * (s + 1)) v[h] = w[h];
+    if (lane / B == s % C) v[s / C] = own[0];
   }
 }
 __device__ __forceinline__ uint64_t gtime() {
@@ -151,7 +159,11 @@ __device__ __forceinline__ uint64_t gtime() {
 }
 
 template <typename T, bool kConj, int kTB = kTBOf<T>, int kTThr = 4 * kTBOf<T>>
-__global__ void __launch_bounds__(kTThr, 1)
+// Two CTAs per SM where the registers allow it: past 148 blocks the CTAs that
+// wait no longer keep later ones out (DTRSV n = 16384: 820 us with one, 610 with
+// two; n = 4096, all resident either way, 106 against 110).  complex128 keeps
+// one: its two tiles take 128 registers.
+__global__ void __launch_bounds__(kTThr, sizeof(T) == 16 ? 1 : 2)
 k_trsv_g(int n, const T* __restrict__ A, size_t lda, T* x, size_t incx, bool lower_eff, bool trans,
          bool unit, unsigned long long* slots, unsigned* ticket, unsigned* done, unsigned* epoch_word,
          unsigned* status, uint64_t limit_ns) {
@@ -159,14 +171,16 @@ k_trsv_g(int n, const T* __restrict__ A, size_t lda, T* x, size_t incx, bool low
   constexpr int W = kWords<T>;
   constexpr int kSlotWords = kTB * W;   // slots per block (<= kTThr)
   extern __shared__ __align__(16) unsigned char smem[];
-  T(*D)[kTB + 1] = reinterpret_cast<T(*)[kTB + 1]>(smem);   // op(A) diagonal block
+  constexpr int kP = kPitchOf<T>;
+  T* D = reinterpret_cast<T*>(smem);   // diagonal block of op(A), in solve order
   // solutions pushed by the earlier CTAs of the cluster: xin[rank][word]
   unsigned long long(*xin)[kSlotWords] =
-      reinterpret_cast<unsigned long long(*)[kSlotWords]>(smem + sizeof(T) * kTB * (kTB + 1));
-  __shared__ T xk[kTB];        // solution of the block being applied
+      reinterpret_cast<unsigned long long(*)[kSlotWords]>(smem + sizeof(T) * kTB * kP);
+  __shared__ __align__(16) T xk[2][kTB + 2 * 4];  // solution of the block being applied (even, odd)
   __shared__ T rv[kTB];        // right-hand side, then this block's solution
+  __shared__ __align__(16) T xs[2 * kCornerOf<T>];
   __shared__ T rdiag[kTB];     // reciprocals of the diagonal
-  __shared__ int abort_flag;
+  __shared__ int gave_up[2];   // a wait of the even / odd block ran out
   __shared__ unsigned sticket, sepoch, my_ticket, my_epoch;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nblk = (n + kTB - 1) / kTB;
@@ -176,7 +190,7 @@ k_trsv_g(int n, const T* __restrict__ A, size_t lda, T* x, size_t incx, bool low
   const int ncl = (int)ncl_u;
   for (int i = tid; i < ncl * kSlotWords; i += kTThr) (&xin[0][0])[i] = 0ull;
   if (tid == 0) {
-    abort_flag = 0;
+    gave_up[0] = gave_up[1] = 0;
     if (rank == 0) {
       // one ticket per cluster: the cluster takes the next ncl blocks in solve
       // order, so it only ever waits for clusters that started earlier
@@ -198,123 +212,141 @@ k_trsv_g(int n, const T* __restrict__ A, size_t lda, T* x, size_t incx, bool low
   auto blk_of = [&](int sp) { return lower_eff ? sp : nblk - 1 - sp; };
   const int blk = active ? blk_of(s) : 0;
   const int b0 = blk * kTB;
+  // row or column of the block <-> its place in the order of the solve
+  auto order_of = [&](int i) { return lower_eff ? i : kTB - 1 - i; };
   auto opv = [](T v) { return kConj ? F::conj(v) : v; };
 
   if (active) {
   // ---- 1. diagonal block, its reciprocals, the row scaling; right-hand side ----
-  for (int e = tid; e < kTB * kTB; e += kTThr) {
-    const int rr = e % kTB, cc = e / kTB;          // stored element (b0 + rr, b0 + cc)
+  constexpr int kQ = kTB / 4;           // columns per thread of a panel tile
+  static_assert(kSlotWords <= kTThr && kTThr == 4 * kTB, "one slot per thread, four threads per row");
+  const int r = (tid >> 3) * 2 + (tid & 1), q = (tid >> 1) & 3;
+  T a[kQ];                              // panel tile, loaded ahead; the diagonal block first
+#pragma unroll
+  for (int u = 0; u < kQ; ++u) {
+    const int rr = tid % kTB, cc = tid / kTB + 4 * u;  // stored element (b0 + rr, b0 + cc)
     const int gr = b0 + rr, gc = b0 + cc;
-    T v = (gr < n && gc < n) ? A[gr + (size_t)gc * lda] : F::zero();
-    const int r = trans ? cc : rr, c = trans ? rr : cc;   // op(A)(r, c)
-    const bool in_tri = lower_eff ? r >= c : r <= c;
-    if (r == c) v = (unit || b0 + r >= n) ? F::one() : opv(v);
-    else v = in_tri ? opv(v) : F::zero();
-    D[r][c] = v;
+    a[u] = (gr < n && gc < n) ? A[gr + (size_t)gc * lda] : F::zero();
   }
-  if (tid < kTB) rv[tid] = (b0 + tid < n) ? x[(size_t)(b0 + tid) * incx] : F::zero();
+  const T rhs = b0 + r < n ? x[(size_t)(b0 + r) * incx] : F::zero();
+  if (tid < kTB) {   // one division per lane; the element comes again from L1
+    const size_t gd = b0 + tid;
+    rdiag[tid] = F::div(F::one(), unit || gd >= (size_t)n ? F::one() : opv(A[gd + gd * lda]));
+  }
   __syncthreads();
-  if (tid < kTB) rdiag[tid] = F::div(F::one(), D[tid][tid]);
-  __syncthreads();
-  for (int e = tid; e < kTB * kTB; e += kTThr) {
-    const int r = e / kTB, c = e % kTB;
-    if (r != c) D[r][c] = F::neg(F::mul(D[r][c], rdiag[r]));
+#pragma unroll
+  for (int u = 0; u < kQ; ++u) {
+    const int rr = tid % kTB, cc = tid / kTB + 4 * u;
+    const int ir = trans ? cc : rr, ic = trans ? rr : cc;   // op(A)(ir, ic)
+    const bool in_tri = lower_eff ? ir > ic : ir < ic;
+    if (ir != ic) D[order_of(ir) * kP + order_of(ic)] = F::neg(F::mul(in_tri ? opv(a[u]) : F::zero(), rdiag[ir]));
   }
 
-  // ---- 2. panel: acc(r) = sum over earlier blocks k of op(A)(b, k) x_k,
-  // in solve order; a block of this cluster is read from the copy its CTA
-  // pushed into this CTA's shared memory, an earlier cluster's from its slots
-  constexpr int kQ = kTB / 4;           // columns per thread of a panel tile
-  static_assert(kSlotWords <= kTThr, "one slot per thread");
-  uint32_t* xkw = reinterpret_cast<uint32_t*>(xk);
-  const int r = tid >> 2, q = tid & 3;
-  T acc = F::zero();
-  for (int idx = 0; idx < s; ++idx) {
-    const int k = blk_of(idx);
-    const int k0 = k * kTB;
-    // thread (r, q) takes columns q * kQ + j of the tile when A is read as
-    // stored (lanes of a warp on 8 consecutive rows of 4 column runs), and
-    // q + 4 j when it is read transposed, where the 4 threads of a row then
-    // read 4 consecutive elements of one stored column (measured: DTRSV T
-    // 221 -> 134-140 us, CTRSV T 221 -> 146-153, ZTRSV T 274 -> 204-216 at
-    // n = 4096).  The tile is held as stored; the conjugation of op C is
-    // applied where an element is used.
-    const bool tcols = trans;
-    T a[kQ];
+  // Panel tile of the block of solve index idx.  Thread (r, q) takes columns
+  // q * kQ + j of the tile when A is read as stored (lanes of a warp on 8
+  // consecutive rows of 4 column runs), and the pairs at 2 q + 8 j when it is
+  // read transposed, where the 4 threads of a row then read 8 consecutive
+  // elements of one stored column (with 16 in a run instead DTRSV T took 1.6
+  // times as long at n = 4096).  The tile is held as stored; the conjugation of
+  // op C is applied where an element is used.
+  auto load_tile = [&](int idx, T (&t)[kQ]) {
+    const int k0 = blk_of(idx) * kTB;
 #pragma unroll
     for (int j = 0; j < kQ; ++j) {
-      const int gr = b0 + r, gc = k0 + (tcols ? q + 4 * j : q * kQ + j);   // op(A)(gr, gc)
+      const int gr = b0 + r, gc = k0 + (trans ? 2 * q + 8 * (j / 2) + j % 2 : q * kQ + j);   // op(A)(gr, gc)
       const bool in = gr < n && gc < n;
-      a[j] = in ? (trans ? A[gc + (size_t)gr * lda] : A[gr + (size_t)gc * lda]) : F::zero();
+      t[j] = in ? (trans ? A[gc + (size_t)gr * lda] : A[gr + (size_t)gc * lda]) : F::zero();
     }
+  };
+
+  bool aborted = false;
+  // ---- 2. panel: sum over earlier blocks k of op(A)(b, k) x_k in solve
+  // order; a block of this cluster is read from the copy its CTA pushed into
+  // this CTA's shared memory, an earlier cluster's from its slots ----
+  T acc[4] = {F::zero(), F::zero(), F::zero(), F::zero()};
+  if (s > 0) load_tile(0, a);
+  for (int idx = 0; idx < s; ++idx) {
+    T ahead[kQ];
+    if (idx + 1 < s) load_tile(idx + 1, ahead);
     if (tid < kSlotWords) {
       const bool local = idx >= s_first;
-      const unsigned long long* sp = local ? &xin[idx - s_first][tid] : slots + (size_t)k * kSlotWords + tid;
+      const unsigned long long* sp =
+          local ? &xin[idx - s_first][tid] : slots + (size_t)blk_of(idx) * kSlotWords + tid;
       unsigned long long w = local ? ld_local_tag(sp) : ld_relaxed_u64(sp);
       if ((unsigned)(w >> 32) != epoch) {
         const uint64_t t0 = gtime();
         for (unsigned spins = 1;; ++spins) {
           w = local ? ld_local_tag(sp) : ld_relaxed_u64(sp);
           if ((unsigned)(w >> 32) == epoch) break;
+          if ((spins & 7u) != 0) continue;
           const uint64_t el = gtime() - t0;
-          if (el > limit_ns || ((spins & 15u) == 0 && el > 20000ull && *(volatile unsigned*)status != 0)) {
+          if (el > limit_ns || ((spins & 63u) == 0 && el > 20000ull && *(volatile unsigned*)status != 0)) {
             atomicOr(status, kStatusTimeout);
-            abort_flag = 1;
+            gave_up[idx & 1] = 1;
             break;
           }
         }
       }
-      xkw[tid] = (uint32_t)w;
+      reinterpret_cast<uint32_t*>(xk[idx & 1])[tid + 2 * W * (tid / (kQ * W))] = (uint32_t)w;
     }
-    __syncthreads();
-    if (abort_flag) break;
+    __syncthreads();  // (the other half of xk is free: every thread passed here after using it)
+    if (gave_up[idx & 1]) {  // (not written again before every thread is past here)
+      aborted = true;
+      break;
+    }
 #pragma unroll
-    for (int j = 0; j < kQ; ++j) F::mac(acc, opv(a[j]), xk[tcols ? q + 4 * j : q * kQ + j]);
-    __syncthreads();
+    for (int j = 0; j < kQ; j += 2) {
+      const Two<T> t = *reinterpret_cast<const Two<T>*>(
+          &xk[idx & 1][trans ? 2 * q + 8 * (j / 2) + 2 * (j / 4) : q * (kQ + 2) + j]);
+      F::mac(acc[j & 3], opv(a[j]), t.x);
+      F::mac(acc[(j & 3) + 1], opv(a[j + 1]), t.y);
+    }
+#pragma unroll
+    for (int j = 0; j < kQ; ++j) a[j] = ahead[j];
   }
-  acc = F::add(acc, F::shfl_xor(acc, 1));
-  acc = F::add(acc, F::shfl_xor(acc, 2));
-  if (q == 0) rv[r] = F::mul(F::sub(rv[r], acc), rdiag[r]);
+  T sum = F::add(F::add(acc[0], acc[1]), F::add(acc[2], acc[3]));
+  sum = F::add(sum, F::shfl_xor(sum, 2));
+  sum = F::add(sum, F::shfl_xor(sum, 4));
+  if (q == 0) rv[r] = F::mul(F::sub(rhs, sum), rdiag[r]);
   __syncthreads();
 
-  // ---- 3. substitution on the row-scaled diagonal block (one warp) ----
-  if (warp == 0 && !abort_flag) {
-    constexpr int R = kRowsPerLaneOf<T>;
-    if constexpr (R == 0) {
-      T v[kTB / 32];
+  // ---- 3. substitution on the row-scaled diagonal block (one warp), its
+  // solution straight into the shared memory of the next CTA ----
+  if (warp == 0) {
+    T v[kTB / 32];
+    int row[kTB / 32];
 #pragma unroll
-      for (int m = 0; m < kTB / 32; ++m) v[m] = rv[lane + 32 * m];
-      if (lower_eff) substitute_strided<T, kTB, true>(D, v, lane);
-      else substitute_strided<T, kTB, false>(D, v, lane);
+    for (int m = 0; m < kTB / 32; ++m) {
+      row[m] = order_of(lane + 32 * m);
+      v[m] = rv[row[m]];
+    }
+    substitute<T, kTB, kCornerOf<T>, kP>(D, xs, v, lane);
+    const bool push = !aborted && (int)rank + 1 < ncl && s + 1 < nblk;
 #pragma unroll
-      for (int m = 0; m < kTB / 32; ++m) rv[lane + 32 * m] = v[m];
-    } else {
-      T v[R];
-      const bool owner = lane < kTB / R;
+    for (int m = 0; m < kTB / 32; ++m) {
+      if (push) {
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(&v[m]);
+        const uint32_t next = tc::mapa_shared(tc::smem_u32(&xin[rank][row[m] * W]), rank + 1);
 #pragma unroll
-      for (int a = 0; a < R; ++a) v[a] = owner ? rv[lane * R + a] : F::zero();
-      if (lower_eff) substitute<T, kTB, R, true>(D, v, lane);
-      else substitute<T, kTB, R, false>(D, v, lane);
-      if (owner) {
-#pragma unroll
-        for (int a = 0; a < R; ++a) rv[lane * R + a] = v[a];
+        for (int w = 0; w < W; ++w) st_cluster_u64(next + 8 * w, ((unsigned long long)epoch << 32) | words[w]);
       }
+      rv[row[m]] = v[m];
     }
   }
   __syncthreads();
 
   // ---- 4. publish: x_b over b, every word of it into the shared memory of
-  // the later CTAs of the cluster (the next one first) and into the block's
-  // slots for later clusters ----
-  if (!abort_flag) {
+  // the CTAs of the cluster after the next one and into the block's slots for
+  // later clusters ----
+  if (!aborted) {
     if (tid < kTB && b0 + tid < n) x[(size_t)(b0 + tid) * incx] = rv[tid];
     if (tid < kSlotWords) {
       const unsigned long long val =
           ((unsigned long long)epoch << 32) | reinterpret_cast<const uint32_t*>(rv)[tid];
       const uint32_t mine = tc::smem_u32(&xin[rank][tid]);
-      for (int d = (int)rank + 1; d < ncl && s_first + d < nblk; ++d)
-        st_cluster_u64(tc::mapa_shared(mine, (uint32_t)d), val);
       st_relaxed_u64(slots + (size_t)blk * kSlotWords + tid, val);
+      for (int d = (int)rank + 2; d < ncl && s_first + d < nblk; ++d)
+        st_cluster_u64(tc::mapa_shared(mine, (uint32_t)d), val);
     }
   }
   }  // active
@@ -365,7 +397,7 @@ coral_status_t trsv_g(Handle* H, int uplo, int trans, int diag, size_t n, const 
   const bool t = trans != CORAL_NO_TRANSPOSE;
   const bool cj = trans == CORAL_CONJ_TRANSPOSE && !std::is_same<T, double>::value;
   const bool lower_eff = (uplo == CORAL_LOWER) != t;
-  const size_t smem = (size_t)kTB * (kTB + 1) * sizeof(T) + (size_t)kDczClMax * kTB * kWords<T> * 8;
+  const size_t smem = (size_t)kTB * kPitchOf<T> * sizeof(T) + (size_t)kDczClMax * kTB * kWords<T> * 8;
   // per device and kernel form: the attributes are set, and the cluster size
   // (16 where the hardware places it, else 8) is chosen, on the first call
   static int cluster_size[2][64] = {{0}};
