@@ -140,8 +140,15 @@ inline unsigned stream_grid(size_t work, size_t per_block, int sm_count, int blo
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Copies a scalar result produced at device address `src` to `dst` per the
-// pointer mode (host: waits on the stream).
+// Where a kernel puts a scalar result of at most 16 bytes: with results on the
+// host straight into the handle's pinned words, which the device can write,
+// else in `staged` (device memory).  A copy engine's transfer of the 4 to 16
+// bytes would cost its own launch and hand-over on every call.
+inline void* result_slot(Handle* h, void* staged) {
+  return h->pointer_mode == CORAL_POINTER_DEVICE ? staged : h->host_pinned;
+}
+// Delivers a scalar result produced at `src` (a result_slot() or device memory)
+// to `dst` per the pointer mode (host: waits on the stream).
 coral_status_t deliver_result(Handle* h, void* dst, const void* src, size_t bytes);
 
 // Split-BF16 GEMM configuration (tile width BN, split-K factor, and whether a

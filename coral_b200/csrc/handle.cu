@@ -45,7 +45,8 @@ coral_status_t deliver_result(Handle* h, void* dst, const void* src, size_t byte
     CORAL_CUDA(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, h->stream));
     return CORAL_OK;
   }
-  CORAL_CUDA(h, cudaMemcpyAsync(h->host_pinned, src, bytes, cudaMemcpyDeviceToHost, h->stream));
+  if (src != h->host_pinned)
+    CORAL_CUDA(h, cudaMemcpyAsync(h->host_pinned, src, bytes, cudaMemcpyDeviceToHost, h->stream));
   CORAL_CUDA(h, cudaStreamSynchronize(h->stream));
   std::memcpy(dst, h->host_pinned, bytes);
   return CORAL_OK;

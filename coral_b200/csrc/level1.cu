@@ -126,6 +126,10 @@ k_dot(size_t n, const float* __restrict__ x, size_t incx, const float* __restric
     for (size_t t = tid; t < n; t += stride) acc += (double)x[t * incx] * y[t * incy];
   }
   double bs = block_sum(acc, sh);
+  if (gridDim.x == 1) {   // nothing to combine
+    if (threadIdx.x == 0) *out = (float)bs;
+    return;
+  }
   if (threadIdx.x == 0) partials[blockIdx.x] = bs;
   if (!last_block(counter)) return;
   double s = 0.0;
@@ -182,6 +186,10 @@ k_iamax(size_t n, const float* __restrict__ x, size_t incx, float* pv,
     }
   }
   ArgBest bb = block_best(best, sh);
+  if (gridDim.x == 1) {   // nothing to combine
+    if (threadIdx.x == 0) *out = (bb.i == ~0ull) ? 0ull : bb.i;
+    return;
+  }
   if (threadIdx.x == 0) { pv[blockIdx.x] = bb.v; pi[blockIdx.x] = bb.i; }
   if (!last_block(counter)) return;
   ArgBest r{-INFINITY, ~0ull};
@@ -292,6 +300,7 @@ coral_status_t coral_sdot(coral_handle_t hh, size_t n, const float* x, size_t in
   if (!y) return bad_arg(H, 4);
   if (incy == 0) return bad_arg(H, 5);
   bool vec = incx == 1 && incy == 1 && aligned16(x) && aligned16(y);
+  dres = static_cast<float*>(result_slot(H, dres));
   unsigned g = stream_grid(n, (size_t)kRedThreads * 8, H->sm_count, 4);
   double* part = static_cast<double*>(scratch(H, g * sizeof(double)));
   if (!part) return CORAL_ERR_ALLOC;
@@ -316,6 +325,7 @@ coral_status_t coral_isamax(coral_handle_t hh, size_t n, const float* x, size_t 
   }
   if (!x) return bad_arg(H, 2);
   bool vec = incx == 1 && aligned16(x);
+  dres = static_cast<unsigned long long*>(result_slot(H, dres));
   unsigned g = stream_grid(n, (size_t)kRedThreads * 8, H->sm_count, 4);
   char* sc = static_cast<char*>(scratch(H, (size_t)g * 16));
   if (!sc) return CORAL_ERR_ALLOC;

@@ -256,6 +256,10 @@ k_dot_x(size_t n, const T* __restrict__ x, size_t incx, const T* __restrict__ y,
   });
   const double br = bsum(ar, sh);
   const double bi = IsCx<T>::v ? bsum(ai, sh) : 0.0;
+  if (gridDim.x == 1) {   // nothing to combine
+    if (threadIdx.x == 0) *out = from2<T>(br, bi);
+    return;
+  }
   if (threadIdx.x == 0) {
     part[2 * blockIdx.x] = br;
     part[2 * blockIdx.x + 1] = bi;
@@ -282,6 +286,10 @@ k_asum_x(size_t n, const T* __restrict__ x, size_t incx, double* part, unsigned*
   double a0 = 0.0;
   visit<T, kUnit>(n, x, incx, nullptr, 0, [&](T u, T, size_t) { a0 += fabs(re_of(u)) + fabs(im_of(u)); });
   const double b = bsum(a0, sh);
+  if (gridDim.x == 1) {   // nothing to combine
+    if (threadIdx.x == 0) *out = (R)b;
+    return;
+  }
   if (threadIdx.x == 0) part[blockIdx.x] = b;
   if (!last_block_l1(counter)) return;
   double s = 0.0;
@@ -422,6 +430,10 @@ k_iamax_x(size_t n, const T* __restrict__ x, size_t incx, double* pv, unsigned l
     if (better(c, best)) best = c;
   });
   const Best bb = bbest(best, sh);
+  if (gridDim.x == 1) {   // nothing to combine
+    if (threadIdx.x == 0) *out = bb.i == ~0ull ? 0ull : bb.i;
+    return;
+  }
   if (threadIdx.x == 0) {
     pv[blockIdx.x] = bb.v;
     pi[blockIdx.x] = bb.i;
@@ -746,6 +758,7 @@ coral_status_t dot_entry(coral_handle_t hh, size_t n, const void* x, size_t incx
   if (!y) return bad_arg(H, 4);
   if (incy == 0) return bad_arg(H, 5);
   if (((uintptr_t)x | (uintptr_t)y) & (align - 1)) return bad_arg(H, 2);
+  dres = static_cast<T*>(result_slot(H, dres));
   double* part = static_cast<double*>(scratch(H, max_l1_blocks(H) * 2 * sizeof(double)));
   if (!part) return CORAL_ERR_ALLOC;
   const T* xx = static_cast<const T*>(x);
@@ -769,6 +782,7 @@ coral_status_t asum_entry(coral_handle_t hh, size_t n, const void* x, size_t inc
   }
   if (!x) return bad_arg(H, 2);
   if ((uintptr_t)x & (align - 1)) return bad_arg(H, 2);
+  dres = static_cast<R*>(result_slot(H, dres));
   double* part = static_cast<double*>(scratch(H, max_l1_blocks(H) * sizeof(double)));
   if (!part) return CORAL_ERR_ALLOC;
   const T* xx = static_cast<const T*>(x);
@@ -791,6 +805,7 @@ coral_status_t nrm2_entry(coral_handle_t hh, size_t n, const void* x, size_t inc
   }
   if (!x) return bad_arg(H, 2);
   if ((uintptr_t)x & (align - 1)) return bad_arg(H, 2);
+  dres = static_cast<R*>(result_slot(H, dres));
   double* part = static_cast<double*>(scratch(H, max_l1_blocks(H) * 2 * sizeof(double)));
   if (!part) return CORAL_ERR_ALLOC;
   unsigned* flag = &H->words->counters[kCtrMisc + 1];
@@ -827,6 +842,7 @@ coral_status_t iamax_entry(coral_handle_t hh, size_t n, const void* x, size_t in
   }
   if (!x) return bad_arg(H, 2);
   if ((uintptr_t)x & (align - 1)) return bad_arg(H, 2);
+  dres = static_cast<unsigned long long*>(result_slot(H, dres));
   char* sc = static_cast<char*>(scratch(H, max_l1_blocks(H) * 16));
   if (!sc) return CORAL_ERR_ALLOC;
   double* pv = reinterpret_cast<double*>(sc);
