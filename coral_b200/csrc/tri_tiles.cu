@@ -10,16 +10,17 @@
 //     stored one -- where CORAL's lda == n fast path walks the triangle column
 //     by column (ssymv.rs:144-211, chemv.rs:142-231); TRMV N uses the row
 //     part, TRMV T the column part;
-//   * diagonal 64 x 64 blocks -- k_tri_tiles: staged in shared memory and
-//     completed there (mirrored for SYMV/HEMV with Re(a_jj) for HEMV,
-//     chemv.rs:179-182; masked to the triangle, unit diagonal = 1, for TRMV);
+//   * diagonal 64 x 64 blocks -- one more CTA per column block of the same
+//     launch, its warps on 16 columns each: the strict triangle in both parts,
+//     a_jj (Re(a_jj) for HEMV, chemv.rs:179-182, 1 for a unit TRMV) once, the
+//     unstored elements not at all;
 //   * k_strip_combine adds, per 32-row strip, its partials in a fixed order
 //     and applies beta (SYMV/HEMV: beta == 0 fills zeros, else multiplies,
 //     ssymv.rs:137-141) or writes x (TRMV).  Results are deterministic.
 //
 // With coral_set_strip_form(CORAL_STRIPS_TMA) an aligned matrix instead takes
 // k_tri_strips_tma, one TMA-fed persistent pass over the whole stored triangle
-// (diagonal blocks included), then the combine: two launches instead of three.
+// (diagonal blocks included), then the combine.
 // On the measured sizes (SSYMV n = 8192, CHEMV n = 4096) it is not faster than
 // the register form, which stays the default.
 #include "common.cuh"
@@ -30,10 +31,6 @@
 
 namespace coral {
 namespace {
-
-constexpr int kT = 64;        // tile edge
-constexpr int kSeg = 8;       // tiles per CTA run
-constexpr int kTriThreads = 256;
 
 enum TriMode { kSymv = 0, kHemv = 1, kTrmvN = 2, kTrmvT = 3, kTrmvC = 4 };
 // Mode traits: which parts a mode uses, and whether the column part (the
@@ -100,128 +97,6 @@ __device__ __forceinline__ float2 scale_x(float2 alpha, float2 x) {
   return make_float2(alpha.x * x.x - alpha.y * x.y, alpha.x * x.y + alpha.y * x.x);
 }
 
-// Index of stored tile (I, J) in packed triangular order.
-__host__ __device__ __forceinline__ size_t tri_index(int I, int J, bool lower) {
-  return lower ? (size_t)I * (I + 1) / 2 + J : (size_t)J * (J + 1) / 2 + I;
-}
-
-template <typename T, int kMode>
-__global__ void __launch_bounds__(kTriThreads)
-k_tri_tiles(int n, const T* __restrict__ A, size_t lda, const T* __restrict__ x, size_t incx,
-            T alpha, bool lower, bool unit, T* __restrict__ rowpart, T* __restrict__ colpart,
-            int max_seg, int diag_only) {
-  constexpr bool kSym = ModeT<kMode>::kSym;
-  constexpr bool kRow = ModeT<kMode>::kRow;
-  constexpr bool kCol = ModeT<kMode>::kCol;
-  // tile[c][r] = element (row r, col c); dynamic, as complex128 tiles pass 48 KB
-  extern __shared__ __align__(16) unsigned char tile_raw[];
-  T(*tile)[kT + 1] = reinterpret_cast<T(*)[kT + 1]>(tile_raw);
-  __shared__ T vJ[kT], vI[kT];
-  __shared__ T red[4][kT];
-
-  const int NT = (n + kT - 1) / kT;
-  const int J = blockIdx.x, seg = blockIdx.y;
-  // Stored tiles of tile-column J: upper I = 0..J, lower I = J..NT-1.
-  const int first = diag_only ? J : (lower ? J : 0);
-  const int count = diag_only ? 1 : (lower ? NT - J : J + 1);
-  const int t0 = seg * kSeg;
-  if (t0 >= count) return;
-  const int t1 = min(count, t0 + kSeg);
-  const int tid = threadIdx.x;
-  const int r = tid % kT, q = tid / kT;  // 4 quarters of 16 columns / rows
-  const int c0 = J * kT;
-
-  if (tid < kT) {
-    const int gc = c0 + tid;
-    T v = gc < n ? x[(size_t)gc * incx] : Cx<T>::zero();
-    vJ[tid] = kSym ? scale_x(alpha, v) : v;
-  }
-  T colacc = Cx<T>::zero();  // column part for column r, quarter q of the rows
-  // Tile elements of this thread (element e = tid + p * 256: row e % 64,
-  // column e / 64), loaded for tile ti+1 while tile ti is computed.
-  constexpr int kPer = kT * kT / kTriThreads;
-  T reg[kPer];
-  auto load_tile = [&](int I) {
-    const int r0 = I * kT;
-#pragma unroll
-    for (int p = 0; p < kPer; ++p) {
-      const int e = tid + p * kTriThreads;
-      const int gr = r0 + e % kT, gc = c0 + e / kT;
-      reg[p] = (gr < n && gc < n) ? __ldcs(A + gr + (size_t)gc * lda) : Cx<T>::zero();
-    }
-  };
-  load_tile(first + t0);
-  for (int ti = t0; ti < t1; ++ti) {
-    const int I = first + ti;
-    const int r0 = I * kT;
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < kPer; ++p) {
-      const int e = tid + p * kTriThreads;
-      tile[e / kT][e % kT] = reg[p];
-    }
-    if (tid < kT) {
-      const int gr = r0 + tid;
-      T v = gr < n ? x[(size_t)gr * incx] : Cx<T>::zero();
-      vI[tid] = kSym ? scale_x(alpha, v) : v;
-    }
-    if (ti + 1 < t1) load_tile(I + 1);
-    __syncthreads();
-    const bool diag = I == J;
-    if (diag) {
-      // Complete the diagonal tile in place: element (rr, cc) with rr, cc in tile.
-      for (int e = tid; e < kT * kT; e += kTriThreads) {
-        const int rr = e % kT, cc = e / kT;
-        const bool stored = lower ? rr >= cc : rr <= cc;
-        if (rr == cc) {
-          if (kMode == kHemv) tile[cc][rr] = Cx<T>::re(tile[cc][rr]);
-          if (ModeT<kMode>::kTr && unit) tile[cc][rr] = Cx<T>::one();
-        } else if (!stored) {
-          if (kSym) {
-            // unstored (rr, cc) = stored (cc, rr), conjugated for HEMV; read
-            // from the stored half, which this pass never overwrites.
-            T s = tile[rr][cc];
-            tile[cc][rr] = kMode == kHemv ? Cx<T>::conj(s) : s;
-          } else {
-            tile[cc][rr] = Cx<T>::zero();
-          }
-        }
-      }
-      __syncthreads();
-    }
-    // Row part: out[r] = sum_c tile(r, c) * vJ[c], quarter q of the columns.
-    if (kRow) {
-      T acc = Cx<T>::zero();
-#pragma unroll
-      for (int c = q * 16; c < q * 16 + 16; ++c) Cx<T>::mac(acc, tile[c][r], vJ[c]);
-      red[q][r] = acc;
-    }
-    // Column part (off-diagonal tiles for SYMV/HEMV; every tile for TRMV T):
-    // out[c = r] += sum_rr conj?(tile(rr, c)) * vI[rr], quarter q of the rows.
-    if (kCol && (!diag || ModeT<kMode>::kColOnly)) {
-#pragma unroll
-      for (int rr = q * 16; rr < q * 16 + 16; ++rr) {
-        T a = tile[r][rr];
-        Cx<T>::mac(colacc, ModeT<kMode>::kConjCol ? Cx<T>::conj(a) : a, vI[rr]);
-      }
-    }
-    __syncthreads();
-    if (kRow && tid < kT) {
-      T s = Cx<T>::add(Cx<T>::add(red[0][tid], red[1][tid]), Cx<T>::add(red[2][tid], red[3][tid]));
-      rowpart[(diag_only ? (size_t)J : tri_index(I, J, lower)) * kT + tid] = s;
-    }
-  }
-  if (kCol) {
-    __syncthreads();
-    red[q][r] = colacc;
-    __syncthreads();
-    if (tid < kT) {
-      T s = Cx<T>::add(Cx<T>::add(red[0][tid], red[1][tid]), Cx<T>::add(red[2][tid], red[3][tid]));
-      colpart[(diag_only ? (size_t)J : ((size_t)J * max_seg + seg)) * kT + tid] = s;
-    }
-  }
-}
-
 __device__ __forceinline__ float beta_apply(float beta, float y) {
   return beta == 0.f ? 0.f : (beta != 1.f ? y * beta : y);
 }
@@ -240,7 +115,7 @@ __device__ __forceinline__ float2 beta_apply(float2 beta, float2 y) {
 }
 
 // ---- register-resident off-diagonal pass ----------------------------------------
-// kC = 64 columns per tile column (the diagonal tile width).  A warp owns a
+// kC = 64 columns per column block.  A warp owns a
 // strip of 32*V rows: each lane V consecutive rows, loaded as one 16-byte
 // vector per column (V = 4 floats or 2 complex; V = 1 when lda or the base
 // are not 16-byte aligned), so a warp load covers a 512-byte contiguous
@@ -300,10 +175,94 @@ template <> struct Vec<float2, 2> {
   static __device__ __forceinline__ void split(const float4& v, float2 (&o)[2]) { o[0] = make_float2(v.x, v.y); o[1] = make_float2(v.z, v.w); }
 };
 
+// The diagonal block of column block J by one CTA: warp w takes columns 16 w ..
+// 16 w + 15, a lane rows lane and lane + 32; row parts are added over the warps in
+// order, then the column part: dsum[J * 64 + i] is the block's share of output i.
+// An element that is not stored takes no part (a zero in its stead would turn an
+// infinite x into NaN).  As a launch of its own on a side stream the blocks cost
+// a fork and a join, and the join kept the combine from launching early: in a
+// plain stream SSYMV of 8192 took 33.0 us and takes 29.3, DSYMV of 64 to 2048
+// 18.4 and 10.2, CHEMV 21.2 and 13.1.  (One warp per block, as a strip: 6 us more
+// at every small n.)
+template <typename T, int kMode>
+__device__ __forceinline__ void diag_block(int n, int J, const T* __restrict__ A, size_t lda, const T* vJ,
+                                           T (*red)[kC], T* __restrict__ dsum, bool lower, bool unit) {
+  constexpr bool kRow = ModeT<kMode>::kRow, kCol = ModeT<kMode>::kCol;
+  constexpr int kP = sizeof(T) >= 8 ? 4 : 8;   // columns in flight (more would cost the strips residency)
+  constexpr int kW = kC / kStripWarps;           // columns per warp
+  __shared__ T cols[kC];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c0 = J * kC;
+  T racc[2] = {Cx<T>::zero(), Cx<T>::zero()};
+#pragma unroll 1
+  for (int h0 = warp * kW; h0 < (warp + 1) * kW; h0 += kP) {
+    T a[kP][2], v[kP];
+#pragma unroll
+    for (int c = 0; c < kP; ++c)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int r = lane + 32 * m, cc = h0 + c;
+        const bool in = (lower ? r >= cc && c0 + r < n : r <= cc) && c0 + cc < n;
+        a[c][m] = in ? __ldcs(A + c0 + r + (size_t)(c0 + cc) * lda) : Cx<T>::zero();
+      }
+#pragma unroll
+    for (int c = 0; c < kP; ++c) {
+      v[c] = Cx<T>::zero();
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int r = lane + 32 * m, cc = h0 + c;
+        const int d = lower ? r - cc : cc - r;   // places off the diagonal
+        T t = a[c][m];
+        if (d == 0 && kMode == kHemv) t = Cx<T>::re(t);
+        if (d == 0 && ModeT<kMode>::kTr && unit) t = Cx<T>::one();
+        T row = racc[m], col = v[c];
+        if (kRow) Cx<T>::mac(row, t, vJ[cc]);
+        if (kCol) Cx<T>::mac(col, ModeT<kMode>::kConjCol ? Cx<T>::conj(t) : t, vJ[r]);
+        if (d >= 0) racc[m] = row;
+        if (d >= (ModeT<kMode>::kColOnly ? 0 : 1)) v[c] = col;
+      }
+    }
+    if (kCol) {
+      // kP values per lane -> one, then over the lanes that share a column
+#pragma unroll
+      for (int o = 16, w = kP / 2; w > 0; o /= 2, w /= 2) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int c = 0; c < w; ++c)
+          v[c] = Cx<T>::add(up ? v[c + w] : v[c], shfl_xor_t(up ? v[c] : v[c + w], o));
+      }
+      T tot = v[0];
+#pragma unroll
+      for (int o = 16 / kP; o > 0; o /= 2) tot = Cx<T>::add(tot, shfl_xor_t(tot, o));
+      if (lane % (32 / kP) == 0) cols[h0 + lane / (32 / kP)] = tot;
+    }
+  }
+  red[warp][lane] = racc[0];
+  red[warp][lane + 32] = racc[1];
+  __syncthreads();
+  const int i = threadIdx.x;
+  if (i < kC) {
+    T t = red[0][i];
+#pragma unroll
+    for (int w = 1; w < kStripWarps; ++w) t = Cx<T>::add(t, red[w][i]);
+    dsum[c0 + i] = kCol ? Cx<T>::add(t, cols[i]) : t;
+  }
+}
+
+// CTAs per SM that the strips' own registers allow; the diagonal block's code
+// must not take more (at two CTAs fewer DTRMV of an unaligned n = 4095 took 17.7
+// us instead of 14.4).
+constexpr int strip_ctas(size_t elem, int mode, int v) {
+  if (elem >= 16) return mode == kHemv ? 4 : 5;
+  if (v > 1) return mode == kSymv || mode == kHemv ? 4 : 5;
+  return elem >= 8 ? (mode == kHemv ? 7 : 8) : 10;
+}
+
 template <typename T, int kMode, int V>
-__global__ void __launch_bounds__(32 * kStripWarps, sizeof(T) >= 16 ? 3 : 4)
+__global__ void __launch_bounds__(32 * kStripWarps, strip_ctas(sizeof(T), kMode, V))
 k_tri_strips(int n, const T* __restrict__ A, size_t lda, const T* __restrict__ x, size_t incx,
-             T alpha, bool lower, T* __restrict__ rowpart, T* __restrict__ colpart, int nsplit) {
+             T alpha, bool lower, bool unit, T* __restrict__ rowpart, T* __restrict__ colpart,
+             T* __restrict__ dsum, int nsplit) {
   constexpr int kS = 32 * V;                 // strip height
   constexpr int kP = 16;                     // columns per pass
   constexpr bool kSym = ModeT<kMode>::kSym;
@@ -320,7 +279,9 @@ k_tri_strips(int n, const T* __restrict__ A, size_t lda, const T* __restrict__ x
   const int s_hi = row_hi > row_lo ? (row_hi + kS - 1) / kS : s_lo;
   // A CTA past its column's last strip leaves at once: it writes no partial
   // (the combine reads only the splits that hold strips).
-  if (s_lo + (int)blockIdx.y * kStripWarps >= s_hi) return;
+  const bool diag = blockIdx.y == 0;
+  const int split = (int)blockIdx.y - 1;
+  if (!diag && s_lo + split * kStripWarps >= s_hi) return;
   if (threadIdx.x < kC) {
     const int gc = c0 + threadIdx.x;
     T v = gc < n ? x[(size_t)gc * incx] : Cx<T>::zero();
@@ -328,8 +289,13 @@ k_tri_strips(int n, const T* __restrict__ A, size_t lda, const T* __restrict__ x
   }
   for (int i = threadIdx.x; i < kStripWarps * kC; i += blockDim.x) (&red[0][0])[i] = Cx<T>::zero();
   __syncthreads();
+  if (diag) {
+    diag_block<T, kMode>(n, J, A, lda, vJ, red, dsum, lower, unit);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    return;
+  }
   // One strip per warp (the grid has enough warps for the longest column).
-  const int gs = s_lo + blockIdx.y * kStripWarps + warp;
+  const int gs = s_lo + split * kStripWarps + warp;
   if (gs < s_hi) {
     const int r0 = gs * kS + lane * V;      // first row of this lane
     bool rv[V];
@@ -411,7 +377,7 @@ k_tri_strips(int n, const T* __restrict__ A, size_t lda, const T* __restrict__ x
       T s = red[0][threadIdx.x];
 #pragma unroll
       for (int w2 = 1; w2 < kStripWarps; ++w2) s = Cx<T>::add(s, red[w2][threadIdx.x]);
-      colpart[((size_t)J * nsplit + blockIdx.y) * kC + threadIdx.x] = s;
+      colpart[((size_t)J * nsplit + split) * kC + threadIdx.x] = s;
     }
   }
   // This CTA's share is written: the combine grid may start launching (its
@@ -768,7 +734,7 @@ template <typename T, int kMode, int V>
 __global__ void __launch_bounds__(32 * kCombineGroups)
 k_strip_combine(int n, T beta, T* __restrict__ y, size_t incy, bool lower,
                 const T* __restrict__ rowpart, const T* __restrict__ colpart, int ncolblk,
-                int nsplit, int folded, const T* __restrict__ drow, const T* __restrict__ dcol) {
+                int nsplit, int folded, const T* __restrict__ dsum) {
   constexpr int kS = 32 * V;
   constexpr bool kRow = ModeT<kMode>::kRow;
   constexpr bool kCol = ModeT<kMode>::kCol;
@@ -829,10 +795,7 @@ k_strip_combine(int n, T beta, T* __restrict__ y, size_t incy, bool lower,
   T t = part[0][lane];
 #pragma unroll
   for (int q = 1; q < kCombineGroups; ++q) t = Cx<T>::add(t, part[q][lane]);
-  if (!folded) {
-    if (kRow) t = Cx<T>::add(t, drow[gr]);
-    if (ModeT<kMode>::kColOnly) t = Cx<T>::add(t, dcol[gr]);
-  }
+  if (!folded) t = Cx<T>::add(t, dsum[gr]);
   T* yp = y + (size_t)gr * incy;
   if (ModeT<kMode>::kTr) *yp = t;
   else *yp = Cx<T>::add(beta_apply(beta, *yp), t);
@@ -850,38 +813,15 @@ coral_status_t launch_strips(Handle* h, int n, const T* A, size_t lda, const T* 
   nsplit = nsplit < 1 ? 1 : (nsplit > 256 ? 256 : nsplit);
   const size_t rp = (size_t)nstrips * ncol * kS;
   const size_t cp = (size_t)ncol * nsplit * kC;
-  const int NT = (n + kT - 1) / kT;  // diagonal tiles (kT == kC)
-  const size_t dlen = (size_t)NT * kT;
-  T* sc = static_cast<T*>(scratch(h, (rp + cp + 2 * dlen) * sizeof(T)));
+  T* sc = static_cast<T*>(scratch(h, (rp + cp + (size_t)ncol * kC) * sizeof(T)));
   if (!sc) return CORAL_ERR_ALLOC;
-  T* drow = sc + rp + cp;
-  T* dcol = drow + dlen;
-  // The diagonal tiles are independent of the strips: run them on the
-  // handle's side stream, forked from and joined back into the main stream.
-  CORAL_CUDA(h, cudaEventRecord(h->fork_event, h->stream));
-  CORAL_CUDA(h, cudaStreamWaitEvent(h->side_stream, h->fork_event, 0));
-  constexpr size_t kTileSmem = (size_t)kT * (kT + 1) * sizeof(T);
-  if (kTileSmem > 48 * 1024) {
-    static uint64_t attr_devices = 0;  // bit d: attribute set on device d
-    const uint64_t bit = h->device < 64 ? (1ull << h->device) : 0;
-    if (!(attr_devices & bit) || !bit) {
-      CORAL_CUDA(h, cudaFuncSetAttribute(k_tri_tiles<T, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTileSmem));
-      attr_devices |= bit;
-    }
-  }
-  k_tri_tiles<T, kMode><<<dim3(NT, 1), kTriThreads, kTileSmem, h->side_stream>>>(n, A, lda, x, incx, alpha,
-                                                                         lower, unit, drow, dcol, 1, 1);
-  coral_status_t s = launch_status(h);
-  if (s != CORAL_OK) return s;
-  CORAL_CUDA(h, cudaEventRecord(h->join_event, h->side_stream));
+  T* dsum = sc + rp + cp;
   timed_begin(h);
-  k_tri_strips<T, kMode, V><<<dim3(ncol, nsplit), 32 * kStripWarps, 0, h->stream>>>(
-      n, A, lda, x, incx, alpha, lower, sc, sc + rp, nsplit);
-  s = launch_status(h);
+  k_tri_strips<T, kMode, V><<<dim3(ncol, nsplit + 1), 32 * kStripWarps, 0, h->stream>>>(
+      n, A, lda, x, incx, alpha, lower, unit, sc, sc + rp, dsum, nsplit);
+  const coral_status_t s = launch_status(h);
   timed_end(h);
   if (s != CORAL_OK) return s;
-  CORAL_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_event, 0));
   // Programmatic dependent launch: the combine's CTAs are scheduled as the
   // strips grid drains instead of after it has fully retired.
   cudaLaunchConfig_t cfg = {};
@@ -896,7 +836,7 @@ coral_status_t launch_strips(Handle* h, int n, const T* A, size_t lda, const T* 
   cfg.numAttrs = 1;
   CORAL_CUDA(h, cudaLaunchKernelEx(&cfg, k_strip_combine<T, kMode, V>, n, beta, y, incy, lower,
                                    static_cast<const T*>(sc), static_cast<const T*>(sc + rp), ncol, nsplit, 0,
-                                   static_cast<const T*>(drow), static_cast<const T*>(dcol)));
+                                   static_cast<const T*>(dsum)));
   return launch_status(h);
 }
 
@@ -959,14 +899,13 @@ coral_status_t launch_strips_tma(Handle* h, int n, const T* A, size_t lda, const
   cfg.numAttrs = 1;
   CORAL_CUDA(h, cudaLaunchKernelEx(&cfg, k_strip_combine<T, kMode, V>, n, beta, y, incy, lower,
                                    static_cast<const T*>(sc), static_cast<const T*>(sc + rp), ncol, nstrips, 1,
-                                   static_cast<const T*>(nullptr), static_cast<const T*>(nullptr)));
+                                   static_cast<const T*>(nullptr)));
   return launch_status(h);
 }
 
 template <typename T, int kMode>
 coral_status_t run_tri_strips(Handle* h, int n, const T* A, size_t lda, const T* x, size_t incx,
                               T alpha, T beta, T* y, size_t incy, bool lower, bool unit) {
-  static_assert(kC == kT, "diagonal tiles are as wide as the tile columns");
   constexpr int V = (int)(16 / sizeof(T));  // one 16-byte vector per lane and column
   const bool vec = aligned16(A) && (lda * sizeof(T)) % 16 == 0;
   if (vec && h->tri_tma) {
