@@ -81,7 +81,7 @@ enum {
 
 /* Kernel form of SYMV / HEMV / TRMV (coral_set_strip_form). */
 enum {
-  CORAL_STRIPS_REGISTER = 0, /* register-streaming strips, diagonal tiles on a side stream, combine */
+  CORAL_STRIPS_REGISTER = 0, /* register-streaming strips and diagonal blocks, combine */
   CORAL_STRIPS_TMA = 1       /* one TMA-fed persistent pass over the whole triangle, combine */
 };
 
