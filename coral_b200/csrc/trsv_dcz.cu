@@ -278,9 +278,8 @@ k_trsv_g(int n, const T* __restrict__ A, size_t lda, T* x, size_t incx, bool low
         for (unsigned spins = 1;; ++spins) {
           w = local ? ld_local_tag(sp) : ld_relaxed_u64(sp);
           if ((unsigned)(w >> 32) == epoch) break;
-          if ((spins & 7u) != 0) continue;
           const uint64_t el = gtime() - t0;
-          if (el > limit_ns || ((spins & 63u) == 0 && el > 20000ull && *(volatile unsigned*)status != 0)) {
+          if (el > limit_ns || ((spins & 15u) == 0 && el > 20000ull && *(volatile unsigned*)status != 0)) {
             atomicOr(status, kStatusTimeout);
             gave_up[idx & 1] = 1;
             break;
