@@ -184,11 +184,14 @@ template <> struct Vec<float2, 2> {
 // plain stream SSYMV of 8192 took 33.0 us and takes 29.3, DSYMV of 64 to 2048
 // 18.4 and 10.2, CHEMV 21.2 and 13.1.  (One warp per block, as a strip: 6 us more
 // at every small n.)
-template <typename T, int kMode>
+template <typename T, int kMode, int V>
 __device__ __forceinline__ void diag_block(int n, int J, const T* __restrict__ A, size_t lda, const T* vJ,
                                            T (*red)[kC], T* __restrict__ dsum, bool lower, bool unit) {
   constexpr bool kRow = ModeT<kMode>::kRow, kCol = ModeT<kMode>::kCol;
-  constexpr int kP = sizeof(T) >= 8 ? 4 : 8;   // columns in flight (more would cost the strips residency)
+  // Columns in flight: all that SYMV / HEMV's vector strips leave registers for (CHEMV
+  // n = 4096 18.7 -> 17.4 us), few where the strips of the form are narrower.
+  constexpr bool kWide = ModeT<kMode>::kSym && (V > 1 || sizeof(T) >= 16);
+  constexpr int kP = kWide ? (sizeof(T) >= 16 ? 8 : 16) : (sizeof(T) >= 8 ? 4 : 8);
   constexpr int kW = kC / kStripWarps;           // columns per warp
   __shared__ T cols[kC];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -290,7 +293,7 @@ k_tri_strips(int n, const T* __restrict__ A, size_t lda, const T* __restrict__ x
   for (int i = threadIdx.x; i < kStripWarps * kC; i += blockDim.x) (&red[0][0])[i] = Cx<T>::zero();
   __syncthreads();
   if (diag) {
-    diag_block<T, kMode>(n, J, A, lda, vJ, red, dsum, lower, unit);
+    diag_block<T, kMode, V>(n, J, A, lda, vJ, red, dsum, lower, unit);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     return;
   }
