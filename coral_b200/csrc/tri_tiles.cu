@@ -175,6 +175,16 @@ template <> struct Vec<float2, 2> {
   static __device__ __forceinline__ void split(const float4& v, float2 (&o)[2]) { o[0] = make_float2(v.x, v.y); o[1] = make_float2(v.z, v.w); }
 };
 
+// x of a column block (times alpha for SYMV / HEMV) into shared memory.
+template <typename T, int kMode>
+__device__ __forceinline__ void stage_x(int n, int c0, const T* __restrict__ x, size_t incx, T alpha, T* vJ) {
+  if (threadIdx.x < kC) {
+    const int gc = c0 + threadIdx.x;
+    T v = gc < n ? x[(size_t)gc * incx] : Cx<T>::zero();
+    vJ[threadIdx.x] = ModeT<kMode>::kSym ? scale_x(alpha, v) : v;
+  }
+}
+
 // The diagonal block of column block J by one CTA: warp w takes columns 16 w ..
 // 16 w + 15, a lane rows lane and lane + 32; row parts are added over the warps in
 // order, then the column part: dsum[J * 64 + i] is the block's share of output i.
@@ -185,7 +195,8 @@ template <> struct Vec<float2, 2> {
 // 18.4 and 10.2, CHEMV 21.2 and 13.1.  (One warp per block, as a strip: 6 us more
 // at every small n.)
 template <typename T, int kMode, int V>
-__device__ __forceinline__ void diag_block(int n, int J, const T* __restrict__ A, size_t lda, const T* vJ,
+__device__ __forceinline__ void diag_block(int n, int J, const T* __restrict__ A, size_t lda,
+                                           const T* __restrict__ x, size_t incx, T alpha, T* vJ,
                                            T (*red)[kC], T* __restrict__ dsum, bool lower, bool unit) {
   constexpr bool kRow = ModeT<kMode>::kRow, kCol = ModeT<kMode>::kCol;
   // Columns in flight: all that SYMV / HEMV's vector strips leave registers for (CHEMV
@@ -197,9 +208,8 @@ __device__ __forceinline__ void diag_block(int n, int J, const T* __restrict__ A
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = J * kC;
   T racc[2] = {Cx<T>::zero(), Cx<T>::zero()};
-#pragma unroll 1
-  for (int h0 = warp * kW; h0 < (warp + 1) * kW; h0 += kP) {
-    T a[kP][2], v[kP];
+  T a[kP][2], v[kP];
+  auto load = [&](int h0) {
 #pragma unroll
     for (int c = 0; c < kP; ++c)
 #pragma unroll
@@ -208,6 +218,13 @@ __device__ __forceinline__ void diag_block(int n, int J, const T* __restrict__ A
         const bool in = (lower ? r >= cc && c0 + r < n : r <= cc) && c0 + cc < n;
         a[c][m] = in ? __ldcs(A + c0 + r + (size_t)(c0 + cc) * lda) : Cx<T>::zero();
       }
+  };
+  load(warp * kW);   // in flight while x is staged
+  stage_x<T, kMode>(n, c0, x, incx, alpha, vJ);
+  __syncthreads();
+#pragma unroll 1
+  for (int h0 = warp * kW; h0 < (warp + 1) * kW; h0 += kP) {
+    if (h0 != warp * kW) load(h0);
 #pragma unroll
     for (int c = 0; c < kP; ++c) {
       v[c] = Cx<T>::zero();
@@ -285,18 +302,14 @@ k_tri_strips(int n, const T* __restrict__ A, size_t lda, const T* __restrict__ x
   const bool diag = blockIdx.y == 0;
   const int split = (int)blockIdx.y - 1;
   if (!diag && s_lo + split * kStripWarps >= s_hi) return;
-  if (threadIdx.x < kC) {
-    const int gc = c0 + threadIdx.x;
-    T v = gc < n ? x[(size_t)gc * incx] : Cx<T>::zero();
-    vJ[threadIdx.x] = kSym ? scale_x(alpha, v) : v;
-  }
-  for (int i = threadIdx.x; i < kStripWarps * kC; i += blockDim.x) (&red[0][0])[i] = Cx<T>::zero();
-  __syncthreads();
   if (diag) {
-    diag_block<T, kMode, V>(n, J, A, lda, vJ, red, dsum, lower, unit);
+    diag_block<T, kMode, V>(n, J, A, lda, x, incx, alpha, vJ, red, dsum, lower, unit);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     return;
   }
+  stage_x<T, kMode>(n, c0, x, incx, alpha, vJ);
+  for (int i = threadIdx.x; i < kStripWarps * kC; i += blockDim.x) (&red[0][0])[i] = Cx<T>::zero();
+  __syncthreads();
   // One strip per warp (the grid has enough warps for the longest column).
   const int gs = s_lo + split * kStripWarps + warp;
   if (gs < s_hi) {
