@@ -824,9 +824,9 @@ coral_status_t launch_strips(Handle* h, int n, const T* A, size_t lda, const T* 
   const int ncol = (n + kC - 1) / kC;
   const int nstrips = (n + kS - 1) / kS;
   // CTAs per column block: one strip per warp in the longest column, so no
-  // warp streams more than one strip (CTAs past a short column's end exit)
-  int nsplit = (nstrips + kStripWarps - 1) / kStripWarps;
-  nsplit = nsplit < 1 ? 1 : (nsplit > 256 ? 256 : nsplit);
+  // warp streams more than one strip (CTAs past a short column's end exit).
+  // Not capped: at the largest n accepted, 2^20, this is 8192 of the grid's 65535.
+  const int nsplit = (nstrips + kStripWarps - 1) / kStripWarps;
   const size_t rp = (size_t)nstrips * ncol * kS;
   const size_t cp = (size_t)ncol * nsplit * kC;
   T* sc = static_cast<T*>(scratch(h, (rp + cp + (size_t)ncol * kC) * sizeof(T)));
