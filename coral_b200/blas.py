@@ -64,6 +64,14 @@ class CoralError(RuntimeError):
         super().__init__(msg)
 
 
+def _raw_stream(torch) -> int:
+    """torch's current stream as a cudaStream_t (making the stream object costs 3 us a call).
+    torch.cuda.current_device() initialises CUDA, or raises torch's own error, as current_stream() does."""
+    dev = torch.cuda.current_device()
+    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return get(dev) if get else torch.cuda.current_stream(dev).cuda_stream
+
+
 class Handle:
     """Owns a coral_handle_t bound to a CUDA stream."""
 
@@ -87,9 +95,8 @@ class Handle:
             pass
 
     def bind_current_stream(self) -> None:
-        # the raw handle of torch.cuda.current_stream(): making the stream object costs 3 us a call
-        from torch import _C
-        self.lib.coral_set_stream(self.h, C.c_void_p(_C._cuda_getCurrentRawStream(_C._cuda_getDevice())))
+        import torch
+        self.lib.coral_set_stream(self.h, _raw_stream(torch))
 
     def set_gemm_mode(self, mode: int) -> None:
         self.check(self.lib.coral_set_gemm_mode(self.h, int(mode)), "coral_set_gemm_mode")
