@@ -30,6 +30,8 @@ SIGNATURES = {
     "coral_create": [C.POINTER(_h)],
     "coral_destroy": [_h],
     "coral_set_stream": [_h, _vp],
+    "coral_bind_stream": [_h, _vp, _i],
+    "coral_mark_stream": [_h],
     "coral_get_stream": [_h, C.POINTER(_vp)],
     "coral_set_pointer_mode": [_h, _i],
     "coral_set_gemm_mode": [_h, _i],

@@ -82,6 +82,7 @@ class Handle:
         if st != 0:
             raise CoralError(st, "coral_create")
         self.h = h
+        self._raw, self._lasts = None, True   # the stream bound last
 
     def close(self) -> None:
         if self.h:
@@ -95,8 +96,14 @@ class Handle:
             pass
 
     def bind_current_stream(self) -> None:
+        """Calls go to torch's current stream.  On a change of stream the handle orders them after
+        the calls before, whose scratch they share."""
         import torch
-        self.lib.coral_set_stream(self.h, _raw_stream(torch))
+        raw = _raw_stream(torch)
+        if raw != self._raw:
+            # an external stream may be destroyed by its owner before the next call: see call()
+            self._raw, self._lasts = raw, raw == 0 or torch.cuda.current_stream().stream_id != raw
+        self.lib.coral_bind_stream(self.h, raw, self._lasts)
 
     def set_gemm_mode(self, mode: int) -> None:
         self.check(self.lib.coral_set_gemm_mode(self.h, int(mode)), "coral_set_gemm_mode")
@@ -160,6 +167,8 @@ class Handle:
     def call(self, name: str, *args) -> None:
         self.bind_current_stream()
         self.check(getattr(self.lib, name)(self.h, *args), name)
+        if not self._lasts:
+            self.lib.coral_mark_stream(self.h)
 
 
 _tls = threading.local()

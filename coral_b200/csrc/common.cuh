@@ -29,6 +29,14 @@ struct Handle {
   int device = 0;
   int sm_count = kNumSMs;
   cudaStream_t stream = nullptr;
+  bool stream_lasts = false;   // bound as one that still exists at the next binding
+  // The calls of a handle share its scratch, arrival counters and TRSV slots: the
+  // stream that used them last, whether an event may still be recorded on it, and
+  // the mark recorded there in advance (see own_state()).
+  cudaStream_t state_stream = nullptr;
+  bool state_used = false, state_lasts = false, state_marked = false;
+  unsigned long long mark_capture = 0;   // capture the mark was recorded in, 0: none
+  cudaEvent_t order_event = nullptr, order_event_captured = nullptr;
   int pointer_mode = CORAL_POINTER_HOST;
   int gemm_mode = CORAL_GEMM_NATIVE;
   uint64_t wait_limit = kDefaultWaitLimit;
@@ -101,6 +109,11 @@ static_assert(sizeof(DeviceWords) == 1024, "DeviceWords layout");
 
 enum CounterSlot { kCtrDot = 0, kCtrNrm2 = 1, kCtrIamax = 2, kCtrGemv = 3, kCtrTrsv = 4,
                    kCtrSymv = 5, kCtrMisc = 6 };
+
+// Called before work on the handle's shared device state is enqueued (scratch()
+// does it): if that state was last used on another stream, the handle's stream
+// waits for what is enqueued there.  Nothing to do on the same stream.
+void own_state(Handle* h);
 
 // Ensure the handle owns at least `bytes` of scratch; returns nullptr on failure.
 void* scratch(Handle* h, size_t bytes);

@@ -19,7 +19,43 @@ coral_status_t cuda_status(Handle* h, cudaError_t err) {
   return CORAL_ERR_CUDA;
 }
 
+// The capture that `s` takes part in, 0 when it is not capturing, ~0 when that
+// cannot be told (the legacy stream beside a capture).
+static unsigned long long capture_of(cudaStream_t s) {
+  if (s == nullptr || s == cudaStreamLegacy) return 0;   // never captured
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(s, &st, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return ~0ull;
+  }
+  return st == cudaStreamCaptureStatusNone ? 0 : id;
+}
+
+// An event is recorded on the last user's stream and waited for on this one, but
+// only if that stream is known to exist still (a destroyed one must not be
+// touched), and only outside of captures or inside the same one: a dependency
+// across the edge of a capture is not allowed, and such calls are ordered by
+// whoever captures and replays.
+void own_state(Handle* h) {
+  if (h->state_used && h->state_stream != h->stream && (h->state_lasts || h->state_marked)) {
+    const unsigned long long now = capture_of(h->stream);
+    const unsigned long long then = h->state_marked ? h->mark_capture : capture_of(h->state_stream);
+    if (now == then && now != ~0ull) {
+      const cudaEvent_t e = now ? h->order_event_captured : h->order_event;
+      if ((h->state_marked || cudaEventRecord(e, h->state_stream) == cudaSuccess))
+        cudaStreamWaitEvent(h->stream, e, 0);
+      cudaGetLastError();
+    }
+  }
+  h->state_stream = h->stream;
+  h->state_used = true;
+  h->state_lasts = h->stream_lasts;
+  h->state_marked = false;
+}
+
 void* scratch(Handle* h, size_t bytes) {
+  own_state(h);
   if (bytes <= h->scratch_bytes) return h->scratch;
   // Round up to 64 MiB granules past the first 16 MiB to avoid re-allocation churn.
   size_t want = bytes < (16u << 20) ? (16u << 20) : ((bytes + (64u << 20) - 1) & ~size_t((64u << 20) - 1));
@@ -67,10 +103,14 @@ static coral_status_t create_handle(Handle** out) {
       cudaMemset(h->words, 0, sizeof(DeviceWords)) != cudaSuccess ||
       cudaMalloc(&h->counters, kCounterPool * sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(h->counters, 0, kCounterPool * sizeof(unsigned)) != cudaSuccess ||
-      cudaMallocHost(&h->host_pinned, 64) != cudaSuccess) {
+      cudaMallocHost(&h->host_pinned, 64) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->order_event, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->order_event_captured, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
     if (h->words) cudaFree(h->words);
     if (h->counters) cudaFree(h->counters);
+    if (h->host_pinned) cudaFreeHost(h->host_pinned);
+    if (h->order_event) cudaEventDestroy(h->order_event);
     delete h;
     return CORAL_ERR_ALLOC;
   }
@@ -113,6 +153,8 @@ static void destroy_handle(Handle* h) {
   if (h->counters) cudaFree(h->counters);
   if (h->trsv_slots) cudaFree(h->trsv_slots);
   if (h->host_pinned) cudaFreeHost(h->host_pinned);
+  if (h->order_event) cudaEventDestroy(h->order_event);
+  if (h->order_event_captured) cudaEventDestroy(h->order_event_captured);
   delete h;
 }
 
@@ -184,6 +226,25 @@ coral_status_t coral_destroy(coral_handle_t handle) {
 coral_status_t coral_set_stream(coral_handle_t handle, void* stream) {
   CORAL_HANDLE(handle);
   H->stream = reinterpret_cast<cudaStream_t>(stream);
+  H->stream_lasts = false;
+  return CORAL_OK;
+}
+
+coral_status_t coral_bind_stream(coral_handle_t handle, void* stream, int lasts) {
+  CORAL_HANDLE(handle);
+  H->stream = reinterpret_cast<cudaStream_t>(stream);
+  H->stream_lasts = lasts != 0;
+  return CORAL_OK;
+}
+
+coral_status_t coral_mark_stream(coral_handle_t handle) {
+  CORAL_HANDLE(handle);
+  if (!H->state_used || H->state_stream != H->stream) return CORAL_OK;
+  const unsigned long long id = capture_of(H->stream);
+  if (id == ~0ull) return CORAL_OK;
+  CORAL_CUDA(H, cudaEventRecord(id ? H->order_event_captured : H->order_event, H->stream));
+  H->mark_capture = id;
+  H->state_marked = true;
   return CORAL_OK;
 }
 

@@ -971,6 +971,7 @@ coral_status_t rotg_entry(coral_handle_t hh, R* a, R* b, R* c, R* s) {
     k_rotg<R><<<1, 1, 0, H->stream>>>(a, b, c, s);
     return launch_status(H);
   }
+  own_state(H);
   R* d = reinterpret_cast<R*>(stage(H));
   const R in[2] = {*a, *b};
   CORAL_CUDA(H, cudaMemcpyAsync(d, in, sizeof(in), cudaMemcpyHostToDevice, H->stream));
@@ -993,6 +994,7 @@ coral_status_t rotmg_entry(coral_handle_t hh, R* d1, R* d2, R* x1, R y1, R* para
     k_rotmg<R><<<1, 1, 0, H->stream>>>(d1, d2, x1, y1, param);
     return launch_status(H);
   }
+  own_state(H);
   R* d = reinterpret_cast<R*>(stage(H));   // d1 d2 x1 | param[5]
   R in[8] = {*d1, *d2, *x1, param[0], param[1], param[2], param[3], param[4]};
   CORAL_CUDA(H, cudaMemcpyAsync(d, in, sizeof(in), cudaMemcpyHostToDevice, H->stream));

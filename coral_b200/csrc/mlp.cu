@@ -518,6 +518,7 @@ size_t coral_mlp_param_count(coral_mlp_t mlp) {
 coral_status_t coral_mlp_get_params(coral_mlp_t mlp, float* host, size_t count) {
   Mlp* n = reinterpret_cast<Mlp*>(mlp);
   if (!n || !host || count != n->nparams) return CORAL_ERR_INVALID_ARG;
+  own_state(n->h);
   CORAL_CUDA(n->h, cudaMemcpyAsync(host, n->params, count * sizeof(float), cudaMemcpyDeviceToHost, n->h->stream));
   CORAL_CUDA(n->h, cudaStreamSynchronize(n->h->stream));
   return CORAL_OK;
@@ -526,6 +527,7 @@ coral_status_t coral_mlp_get_params(coral_mlp_t mlp, float* host, size_t count) 
 coral_status_t coral_mlp_set_params(coral_mlp_t mlp, const float* host, size_t count) {
   Mlp* n = reinterpret_cast<Mlp*>(mlp);
   if (!n || !host || count != n->nparams) return CORAL_ERR_INVALID_ARG;
+  own_state(n->h);
   CORAL_CUDA(n->h, cudaMemcpyAsync(n->params, host, count * sizeof(float), cudaMemcpyHostToDevice, n->h->stream));
   CORAL_CUDA(n->h, cudaMemsetAsync(n->adam_m, 0, count * sizeof(float), n->h->stream));
   CORAL_CUDA(n->h, cudaMemsetAsync(n->adam_v, 0, count * sizeof(float), n->h->stream));
@@ -539,6 +541,7 @@ coral_status_t coral_mlp_forward(coral_mlp_t mlp, const float* x, int batch, flo
   if (!n) return CORAL_ERR_INVALID_ARG;
   if (batch < 0 || (batch > 0 && (!x || !y))) return bad_arg(n->h, 2);
   if (batch == 0) return CORAL_OK;
+  own_state(n->h);   // the network's buffers are shared like the handle's
   return forward(n, x, batch, y);
 }
 
@@ -547,6 +550,7 @@ coral_status_t coral_mlp_gradients(coral_mlp_t mlp, const float* x, const float*
   Mlp* n = reinterpret_cast<Mlp*>(mlp);
   if (!n) return CORAL_ERR_INVALID_ARG;
   if (batch < 1 || !x || !target) return bad_arg(n->h, 2);
+  own_state(n->h);
   coral_status_t s = backward(n, x, target, batch);
   if (s != CORAL_OK) return s;
   if (grads)
@@ -563,6 +567,7 @@ coral_status_t coral_mlp_train_step(coral_mlp_t mlp, const float* x, const float
   Mlp* n = reinterpret_cast<Mlp*>(mlp);
   if (!n) return CORAL_ERR_INVALID_ARG;
   if (batch < 1 || !x || !target) return bad_arg(n->h, 2);
+  own_state(n->h);
   coral_status_t s = backward(n, x, target, batch);
   if (s != CORAL_OK) return s;
   n->step += 1;

@@ -822,6 +822,7 @@ extern "C" coral_status_t coral_strsv(coral_handle_t hh, int uplo, int trans, in
   constexpr int nb = 64;
   const size_t nblk = (n + nb - 1) / nb;
   if (n > (size_t)INT32_MAX) return CORAL_ERR_NOT_SUPPORTED;
+  own_state(H);
   if (H->trsv_slots_len < nblk * nb) {
     if (H->trsv_slots) {
       CORAL_CUDA(H, cudaStreamSynchronize(H->stream));

@@ -381,6 +381,7 @@ coral_status_t trsv_g(Handle* H, int uplo, int trans, int diag, size_t n, const 
   constexpr int kTB = kTBOf<T>, kTThr = 4 * kTBOf<T>;
   const size_t nblk = (n + kTB - 1) / kTB;
   const size_t nslots = nblk * kTB * kWords<T>;   // one slot per 32-bit word of x
+  own_state(H);
   if (H->trsv_slots_len < nslots) {
     if (H->trsv_slots) {
       CORAL_CUDA(H, cudaStreamSynchronize(H->stream));

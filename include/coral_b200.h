@@ -94,8 +94,21 @@ typedef struct coral_handle_s* coral_handle_t;
  * waits set, and the per-handle configuration. */
 coral_status_t coral_create(coral_handle_t* handle);
 coral_status_t coral_destroy(coral_handle_t handle);
-/* `stream` is a cudaStream_t (NULL = legacy default stream). */
+/* `stream` is a cudaStream_t (NULL = legacy default stream).  Calls of one handle
+ * share its scratch: after a change of stream with coral_set_stream, calls on the
+ * new stream are ordered after those on the old one by the caller (or take one
+ * handle per stream). */
 coral_status_t coral_set_stream(coral_handle_t handle, void* stream);
+/* The same, with that ordering done by the handle: the first call that uses the
+ * shared scratch on another stream waits, on the device, for the stream that used
+ * it last.  `lasts` != 0 promises that `stream` still exists when that happens;
+ * with 0 only calls up to the last coral_mark_stream are waited for.  Nothing is
+ * ordered across the edge of a stream capture: a captured call is ordered where
+ * its graph is launched. */
+coral_status_t coral_bind_stream(coral_handle_t handle, void* stream, int lasts);
+/* Records the point up to which the next call on another stream waits, so that the
+ * handle's stream may be destroyed afterwards. */
+coral_status_t coral_mark_stream(coral_handle_t handle);
 coral_status_t coral_get_stream(coral_handle_t handle, void** stream);
 coral_status_t coral_set_pointer_mode(coral_handle_t handle, int mode);
 coral_status_t coral_set_gemm_mode(coral_handle_t handle, int mode);

@@ -52,3 +52,15 @@ def test_without_the_raw_getter(monkeypatch, fake_cuda):
     h = _handle()
     h.bind_current_stream()
     assert h.lib.calls[-1][2] == 0x7f0010
+
+
+def test_only_external_streams_are_marked(fake_cuda):
+    h = _handle()
+    for stream, lasts in ((FakeStream(0, 0), True), (FakeStream(35, 0x7f0010), True),
+                          (FakeStream(0x7f0020, 0x7f0020), False), (FakeStream(35, 0x7f0010), True)):
+        fake_cuda["stream"] = stream
+        h.lib.calls.clear()
+        h.call("coral_saxpy", 1)
+        names = [c[0] for c in h.lib.calls]
+        assert h.lib.calls[0] == ("coral_bind_stream", None, stream.cuda_stream, lasts)
+        assert names == ["coral_bind_stream", "coral_saxpy"] + ([] if lasts else ["coral_mark_stream"])
