@@ -730,7 +730,7 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
       for (int j = 0; j < kCols; ++j) sum[j] = 0.f;
       for (int c = 0; c < chunks; ++c, ++gc) {
         const int b = gc & 1;
-        if (!tc::mbar_wait(&chunk_full[b], (gc >> 1) & 1, limit_ns)) {
+        if (!tc::mbar_wait_warp(&chunk_full[b], (gc >> 1) & 1, limit_ns)) {
           atomicOr(status, kStatusTimeout);
           stop = true;
           break;
@@ -750,7 +750,7 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&chunk_empty[b]);
       }
-      if (stop || *(volatile int*)&abort_flag) break;
+      if (stop || tc::flag_warp(&abort_flag)) break;
       const int row = t.mt * kBM + quad * 32 + lane;
       if (row >= ep.m) continue;
       const int col0 = t.col0 + half * ncols;  // first accumulator column of this thread
@@ -980,7 +980,7 @@ k_gemm_split_pair(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles,
       for (int j = 0; j < kCols; ++j) sum[j] = 0.f;
       for (int c = 0; c < chunks; ++c, ++gc) {
         const int b = gc & 1;
-        if (!tc::mbar_wait(&chunk_full[b], (gc >> 1) & 1, limit_ns)) {
+        if (!tc::mbar_wait_warp(&chunk_full[b], (gc >> 1) & 1, limit_ns)) {
           atomicOr(status, kStatusTimeout);
           stop = true;
           break;
@@ -999,7 +999,7 @@ k_gemm_split_pair(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles,
         __syncwarp();
         if (lane == 0) tc::mbar_arrive_cluster(tc::mapa_shared(tc::smem_u32(&chunk_empty[b]), 0));
       }
-      if (stop || *(volatile int*)&abort_flag) break;
+      if (stop || tc::flag_warp(&abort_flag)) break;
       const int row = mt * kPairTile + (int)rank * kPairHalf + quad * 32 + lane;
       if (row >= ep.m) continue;
       const int col0 = nt * kPairTile + half * kCols;

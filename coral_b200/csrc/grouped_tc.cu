@@ -396,14 +396,15 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
     atomicExch(&abort_flag, 1);
   };
   // Consumer side of the tile queue: the j-th tile of this CTA, which stays valid
-  // until release_tile(j) (one arrival per consumer warp).
-  auto next_tile = [&](int j) -> const TileInfo* {
+  // until release_tile(j) (one arrival per consumer warp).  A whole warp calls it,
+  // all of its lanes with the same answer (see mbar_wait_warp), or one lane.
+  auto next_tile = [&](int j, bool whole_warp) -> const TileInfo* {
     const int q = j % kQueue;
-    if (!tc::mbar_wait(&tq_full[q], (j / kQueue) & 1, limit_ns)) {
-      give_up();
-      return nullptr;
-    }
-    return tq[q].more && !*(volatile int*)&abort_flag ? &tq[q] : nullptr;
+    bool go = tc::mbar_wait(&tq_full[q], (j / kQueue) & 1, limit_ns);
+    if (!go) give_up();
+    go = go && !*(volatile int*)&abort_flag;
+    if (whole_warp) go = __all_sync(0xffffffffu, go);
+    return go && tq[q].more ? &tq[q] : nullptr;
   };
   auto release_tile = [&](int j) { tc::mbar_arrive(&tq_empty[j % kQueue]); };
 
@@ -458,7 +459,7 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
     int it0 = 0;  // running number of the tile's first slab
     bool stop = false;
     const TileInfo* tp;
-    for (int j = 0; !stop && (tp = next_tile(j)); ++j) {
+    for (int j = 0; !stop && (tp = next_tile(j, true)); ++j) {
       const TileInfo& ti = *tp;
       const coral_sgemm_problem_t& p = ti.p;
       // C is read in the epilogue, a column at a time: bring it into L2 now
@@ -487,7 +488,7 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
 #pragma unroll
             for (int u = 0; u < kInFlight; ++u)
               if (b0 + u < nb) o.load(b0 + u, left, tid, v[u]);
-            if (b0 == 0 && it >= S && !tc::mbar_wait(&empty_bar[s], ((it / S) - 1) & 1, limit_ns)) {
+            if (b0 == 0 && it >= S && !tc::mbar_wait_warp(&empty_bar[s], ((it / S) - 1) & 1, limit_ns)) {
               give_up();
               stop = true;
               break;
@@ -512,7 +513,7 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
       int it = 0, gc = 0;
       bool stop = false;
       const TileInfo* tp;
-      for (int j = 0; !stop && (tp = next_tile(j)); ++j) {
+      for (int j = 0; !stop && (tp = next_tile(j, false)); ++j) {
         const int nslabs = tp->nslabs;
         const uint32_t idesc = tc::idesc_bf16_f32(kTM, tp->bn);
         release_tile(j);
@@ -570,7 +571,7 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
     int gc = 0;
     bool stop = false;
     const TileInfo* tp;
-    for (int j = 0; !stop && (tp = next_tile(j)); ++j) {
+    for (int j = 0; !stop && (tp = next_tile(j, true)); ++j) {
       const int m0 = tp->m0, n0 = tp->n0, nslabs = tp->nslabs, m = tp->p.m;
       const int row = m0 + quad * 32 + lane;
       const int ncols = min(tp->bn, tp->p.n - n0);
@@ -613,7 +614,7 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
         };
         // the first 16 columns of C on their way while the products finish
         load_c(q, ncols - 16 * half);
-        if (!tc::mbar_wait(&acc_full[b], (gc >> 1) & 1, limit_ns)) {
+        if (!tc::mbar_wait_warp(&acc_full[b], (gc >> 1) & 1, limit_ns)) {
           give_up();
           stop = true;
           break;

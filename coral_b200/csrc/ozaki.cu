@@ -488,7 +488,7 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
     const uint64_t ring = tc::desc_k_sw64(tc::smem_u32(smem));
     const uint32_t ring_lo = (uint32_t)ring, hi = (uint32_t)(ring >> 32);
     auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-      if (__all_sync(0xffffffffu, tc::mbar_wait(bar, parity, limit_ns))) return true;
+      if (tc::mbar_wait_warp(bar, parity, limit_ns)) return true;
       if (lead) {
         atomicOr(status, kStatusTimeout);
         atomicExch(&abort_flag, 1);
@@ -569,7 +569,7 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
       for (int c0 = 0; c0 < nk && !stop; c0 += chunk_kb) {
 #pragma unroll
         for (int pass = 0; pass < P::kPasses; ++pass, ++gc) {
-          if (stop || !tc::mbar_wait(&acc_full, gc & 1, limit_ns)) {
+          if (stop || !tc::mbar_wait_warp(&acc_full, gc & 1, limit_ns)) {
             atomicOr(status, kStatusTimeout);
             stop = true;
             break;
@@ -589,7 +589,7 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
           if (lane == 0) tc::mbar_arrive(&acc_empty);
         }
       }
-      if (stop || *(volatile int*)&abort_flag) break;
+      if (stop || tc::flag_warp(&abort_flag)) break;
       const int row = mt * kOzBM + quad * 32 + lane;
       if (row >= ep.m) continue;
       const int ei = max(ep.ea[row], -4000);  // all-zero rows keep the INT_MIN-like fill

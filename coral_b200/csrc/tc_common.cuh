@@ -73,6 +73,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
   return false;
 }
 
+// The same for a whole warp, with one answer for all of its lanes: each lane gives up
+// by its own reading of the timer, and lanes that left a loop alone would meet the
+// CTA's barrier while the others stand at a __syncwarp or a warp-wide instruction.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit_ns));
+}
+// Whether a flag in shared memory is set, with one answer for the warp.
+__device__ __forceinline__ bool flag_warp(const int* flag) {
+  return __any_sync(0xffffffffu, *(const volatile int*)flag);
+}
+
 // 2-D tiled TMA load into this CTA's shared memory, completing on `bar`.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar,
                                             int32_t c0, int32_t c1) {

@@ -682,8 +682,8 @@ k_tri_strips_tma(const __grid_constant__ CUtensorMap map, int n, const T* __rest
       if (i + kTsGroups < share.count)
         unit_x<T, kMode, V>(walk, share.unit(i + kTsGroups), n, lower, x, incx, cw, lane, nx);
       const int st = i % kTsStages;
-      bool ok = !*(volatile int*)&abort_flag;
-      if (ok && !tc::mbar_wait(&full_bar[st], (i / kTsStages) & 1, limit_ns)) {
+      bool ok = !tc::flag_warp(&abort_flag);
+      if (ok && !tc::mbar_wait_warp(&full_bar[st], (i / kTsStages) & 1, limit_ns)) {
         atomicOr(status, kStatusTimeout);
         atomicExch(&abort_flag, 1);
         ok = false;

@@ -569,7 +569,7 @@ k_trsv_cluster(const __grid_constant__ CUtensorMap amap, int n, float* x, size_t
     // ---------------- consumer warps ----------------
     // the right-hand side is read first so its latency hides behind the wait
     const float rhs_v = (tid < kCB && b0 + tid < n) ? x[(size_t)(b0 + tid) * incx] : 0.f;
-    bool ok = tc::mbar_wait(&S.setup_bar, 0, limit_ns);
+    bool ok = tc::mbar_wait_warp(&S.setup_bar, 0, limit_ns);
     // op(D) masked: stored element (b0 + rr, b0 + cc) sits at raw[0][cc][rr].
     // An upper op(D) is stored index-reversed (L = P op(D) P, P the reversal),
     // which is lower triangular, and so are the rows of the right-hand sides.
