@@ -574,7 +574,7 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = tc::align1024_shared(smem_raw);
   __shared__ __align__(8) uint64_t full_bar[kStages], empty_bar[kStages];
-  __shared__ __align__(8) uint64_t chunk_full[2], chunk_empty[2];
+  __shared__ __align__(8) uint64_t chunk_full[2], chunk_empty[2], drain_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -610,6 +610,7 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
       tc::mbar_init(&chunk_full[b], 1);
       tc::mbar_init(&chunk_empty[b], kEpiWarps);
     }
+    tc::mbar_init(&drain_bar, 1);
     abort_flag = 0;
     tc::fence_mbar_init();
   }
@@ -662,7 +663,7 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
       }
       // Drain: every issued load lands before the CTA may exit.
       for (int j = (it > kStages ? it - kStages : 0); j < it; ++j)
-        tc::mbar_wait(&full_bar[j % kStages], (j / kStages) & 1, limit_ns);
+        tc::mbar_wait(&full_bar[j % kStages], (j / kStages) & 1, tc::kDrainNs);
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -710,6 +711,9 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
           tc::mma_commit(&chunk_full[b]);
         }
       }
+      // every product issued completes before TMEM is released
+      tc::mma_commit(&drain_bar);
+      tc::mbar_wait(&drain_bar, 0, tc::kDrainNs);
     }
   } else {
     // ---- epilogue warps ----
@@ -840,7 +844,7 @@ k_gemm_split_pair(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles,
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = tc::align1024_shared(smem_raw);
   __shared__ __align__(8) uint64_t full_bar[kS], empty_bar[kS];
-  __shared__ __align__(8) uint64_t chunk_full[2], chunk_empty[2];
+  __shared__ __align__(8) uint64_t chunk_full[2], chunk_empty[2], drain_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -865,6 +869,7 @@ k_gemm_split_pair(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles,
       tc::mbar_init(&chunk_full[b], 1);
       tc::mbar_init(&chunk_empty[b], 2 * kEpiWarps);
     }
+    tc::mbar_init(&drain_bar, 1);
     abort_flag = 0;
     tc::fence_mbar_init();
   }
@@ -914,7 +919,7 @@ k_gemm_split_pair(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles,
       // Drain: a slab's loads have landed once the MMA that read it released
       // the slot, so wait for the last slots' releases before exiting.
       for (int j = (it > kS ? it - kS : 0); j < it; ++j)
-        tc::mbar_wait(&empty_bar[j % kS], (j / kS) & 1, limit_ns);
+        tc::mbar_wait(&empty_bar[j % kS], (j / kS) & 1, tc::kDrainNs);
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
@@ -961,6 +966,9 @@ k_gemm_split_pair(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles,
           tc::mma_commit_pair(&chunk_full[b], kPairMask);
         }
       }
+      // every product issued completes before either CTA releases TMEM
+      tc::mma_commit_pair(&drain_bar, 1);
+      tc::mbar_wait(&drain_bar, 0, tc::kDrainNs);
     }
   } else {
     // ---- epilogue warps (both CTAs): rows [128 r, 128 r + 128) of the tile ----

@@ -560,9 +560,8 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
         }
       }
       // every MMA issued by this thread completes before TMEM is released
-      // (own 1 s bound: the configured limit may be tiny)
       tc::mma_commit(&drain_bar);
-      tc::mbar_wait(&drain_bar, 0, 1000000000ull);
+      tc::mbar_wait(&drain_bar, 0, tc::kDrainNs);
     }
   } else {
     // ---- epilogue ----

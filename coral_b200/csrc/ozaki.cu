@@ -403,7 +403,7 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = tc::align1024_shared(smem_raw);
   __shared__ __align__(8) uint64_t full_bar[kSlots], empty_bar[kSlots];
-  __shared__ __align__(8) uint64_t acc_full, acc_empty;
+  __shared__ __align__(8) uint64_t acc_full, acc_empty, drain_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -418,6 +418,7 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
     }
     tc::mbar_init(&acc_full, 1);
     tc::mbar_init(&acc_empty, kOzEpiWarps);
+    tc::mbar_init(&drain_bar, 1);
     abort_flag = 0;
     tc::fence_mbar_init();
   }
@@ -476,9 +477,9 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
           }
         }
       }
-      // every issued load lands before the CTA may exit (own 1 s bound)
+      // every issued load lands before the CTA may exit
       for (int j = (it > kSlots ? it - kSlots : 0); j < it; ++j)
-        tc::mbar_wait(&full_bar[j % kSlots], (j / kSlots) & 1, 1000000000ull);
+        tc::mbar_wait(&full_bar[j % kSlots], (j / kSlots) & 1, tc::kDrainNs);
     }
   } else if (warp == 1) {
     // ---- MMA issuer: the warp stays converged, one lane issues ----
@@ -543,6 +544,11 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
         }
       }
     }
+    if (lead) {  // every product issued completes before TMEM is released
+      tc::mma_commit(&drain_bar);
+      tc::mbar_wait(&drain_bar, 0, tc::kDrainNs);
+    }
+    __syncwarp();
   } else {
     const int ew = warp - 2;
     const int quad = warp & 3;

@@ -73,6 +73,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
   return false;
 }
 
+// Bound of the waits for copies and products in flight before a CTA leaves: their own,
+// because the caller's limit may be far shorter than a copy.
+constexpr uint64_t kDrainNs = 1000000000ull;
+
 // The same for a whole warp, with one answer for all of its lanes: each lane gives up
 // by its own reading of the timer, and lanes that left a loop alone would meet the
 // CTA's barrier while the others stand at a __syncwarp or a warp-wide instruction.

@@ -666,7 +666,7 @@ k_tri_strips_tma(const __grid_constant__ CUtensorMap map, int n, const T* __rest
       }
       // every issued copy lands before the CTA may exit
       for (int j = (i > kTsStages ? i - kTsStages : 0); j < i; ++j)
-        tc::mbar_wait(&full_bar[j % kTsStages], (j / kTsStages) & 1, 1000000000ull);
+        tc::mbar_wait(&full_bar[j % kTsStages], (j / kTsStages) & 1, tc::kDrainNs);
     }
   } else {
     // ---- consumers: group cg takes the CTA's units cg, cg + 2, ...; warp cw
