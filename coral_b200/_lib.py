@@ -145,6 +145,7 @@ SIGNATURES = {
     "coral_set_gemm_config": [_h, _i, _i],
     "coral_set_gemm_tile": [_h, _i, _i, _i],
     "coral_get_gemm_tile": [_h, _i, _i, _i, _sz, _sz, _sz, C.POINTER(_i), C.POINTER(_i), C.POINTER(_i)],
+    "coral_default_gemm_tile": [_i, _sz, _sz, _sz, _i, C.POINTER(_i), C.POINTER(_i), C.POINTER(_i)],
     "coral_set_pair_raster": [_h, _i],
     "coral_autotune_sgemm_tiles": [_h, _i, _i, _i, _sz, _sz, _sz, _vp, _sz, _vp, _sz, _vp, _sz, _i,
                                    C.POINTER(_f), _i, C.POINTER(_i), C.POINTER(_i)],

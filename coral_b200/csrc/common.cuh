@@ -177,6 +177,8 @@ struct SplitShape {
   int batch;
 };
 SplitConfig choose_split_config(Handle* h, const SplitShape& sh);
+// The rule that applies without an explicit configuration and without a selector.
+SplitConfig default_split_config(int products, int mr, int nr, int kd, int sm_count);
 // Asks the handle's selector for a configuration; false if it has none.
 bool select_split_config(Handle* h, const SplitShape& sh, SplitConfig* out);
 // Features of (shape, configuration) for the selector network.

@@ -1197,14 +1197,43 @@ coral_status_t run_split_gemm_pair(Handle* h, const __nv_bfloat16* ap, size_t a_
 
 }  // namespace
 
-// Tile width and split-K factor for a split-BF16 GEMM of op(A) (mr x kd)
-// times B-rows (nr x kd): the handle's explicit choice, else its selector,
-// else the default rule (256 columns, or 128 where those fill one wave at most or
-// K is short; K in parts when the output tiles cannot fill the GPU and K is deep).
-SplitConfig choose_split_config(Handle* h, const SplitShape& sh) {
-  const int products = sh.products, mr = sh.mr, nr = sh.nr, kd = sh.kd;
+// The default rule: 256 columns, or 128 where those fill one wave at most or K is
+// short; K in parts when the output tiles cannot fill the GPU and K is deep.
+SplitConfig default_split_config(int products, int mr, int nr, int kd, int sm_count) {
   SplitConfig c{products == 3 ? 256 : 128, 1};
   const int nk = (kd + 63) / 64;   // 64-deep K units (independent of the kernel's slab depth)
+  const int m_tiles = (mr + kBM - 1) / kBM;
+  const int tiles = m_tiles * ((nr + c.bn - 1) / c.bn), tiles128 = m_tiles * ((nr + 127) / 128);
+  const int pair_tiles = ((mr + kPairTile - 1) / kPairTile) * ((nr + kPairTile - 1) / kPairTile);
+  if (tiles > 0 && tiles * 2 <= sm_count && nk >= 16) {
+    // split K (its parts also bound how many tensor-core additions a sum goes through)
+    int sp = sm_count / tiles;
+    sp = sp > 16 ? 16 : sp;
+    sp = sp > nk ? nk : sp;
+    int p2 = 1;  // largest power of two <= sp (the tuned candidate set)
+    while (p2 * 2 <= sp) p2 *= 2;
+    c.splits = p2;
+  } else if (tiles128 <= sm_count || (nk <= 5 && products == 3)) {
+    // One wave of 128 x 128 tiles, or a product whose time goes into C: half
+    // the columns per tile are drained and written in half the time (us, 128 /
+    // 256 wide: 700^3 19.5 / 24.7, 1500^3 34.9 / 41.5, 4096 x 4096 x 256 47 / 57).
+    c.bn = 128;
+  } else if (pair_tiles >= sm_count) {
+    // At least two waves of 256 x 256 tiles over the resident CTA pairs:
+    // the pair tiles read half as much of B per flop from shared memory.
+    c.pair = 1;
+    c.bn = 256;
+  }
+  return c;
+}
+
+// Tile width and split-K factor for a split-BF16 GEMM of op(A) (mr x kd)
+// times B-rows (nr x kd): the handle's explicit choice, else its selector,
+// else the default rule.
+SplitConfig choose_split_config(Handle* h, const SplitShape& sh) {
+  const int products = sh.products, kd = sh.kd;
+  SplitConfig c{products == 3 ? 256 : 128, 1};
+  const int nk = (kd + 63) / 64;
   if (h->cfg_bn > 0 || h->cfg_splits > 0 || h->cfg_bm > 0) {
     if (h->cfg_bn > 0) c.bn = h->cfg_bn;
     if (h->cfg_splits > 0) c.splits = h->cfg_splits;
@@ -1212,31 +1241,8 @@ SplitConfig choose_split_config(Handle* h, const SplitShape& sh) {
       c.pair = 1;
       c.bn = 256;
     }
-  } else if (h->selector && select_split_config(h, sh, &c)) {
-    // selector decided
-  } else {
-    const int m_tiles = (mr + kBM - 1) / kBM;
-    const int tiles = m_tiles * ((nr + c.bn - 1) / c.bn), tiles128 = m_tiles * ((nr + 127) / 128);
-    const int pair_tiles = ((mr + kPairTile - 1) / kPairTile) * ((nr + kPairTile - 1) / kPairTile);
-    if (tiles * 2 <= h->sm_count && nk >= 16) {
-      // split K (its parts also bound how many tensor-core additions a sum goes through)
-      int sp = h->sm_count / tiles;
-      sp = sp > 16 ? 16 : sp;
-      sp = sp > nk ? nk : sp;
-      int p2 = 1;  // largest power of two <= sp (the tuned candidate set)
-      while (p2 * 2 <= sp) p2 *= 2;
-      c.splits = p2;
-    } else if (tiles128 <= h->sm_count || (nk <= 5 && products == 3)) {
-      // One wave of 128 x 128 tiles, or a product whose time goes into C: half
-      // the columns per tile are drained and written in half the time (us, 128 /
-      // 256 wide: 700^3 19.5 / 24.7, 1500^3 34.9 / 41.5, 4096 x 4096 x 256 47 / 57).
-      c.bn = 128;
-    } else if (pair_tiles >= h->sm_count) {
-      // At least two waves of 256 x 256 tiles over the resident CTA pairs:
-      // the pair tiles read half as much of B per flop from shared memory.
-      c.pair = 1;
-      c.bn = 256;
-    }
+  } else if (!(h->selector && select_split_config(h, sh, &c))) {
+    c = default_split_config(products, sh.mr, sh.nr, kd, h->sm_count);
   }
   if (products == 6 && !c.pair) c.bn = 128;
   if (c.bn != 128 && c.bn != 256) c.bn = 256;

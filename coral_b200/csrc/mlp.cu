@@ -651,6 +651,18 @@ coral_status_t coral_get_gemm_tile(coral_handle_t hh, int products, int op_a, in
   return CORAL_OK;
 }
 
+coral_status_t coral_default_gemm_tile(int products, size_t m, size_t n, size_t k, int sm_count, int* tile_m,
+                                       int* tile_n, int* split_k) {
+  if ((products != 3 && products != 6) || sm_count < 1 || !tile_m || !tile_n || !split_k)
+    return CORAL_ERR_INVALID_ARG;
+  if (!shape_fits(m, n, k)) return CORAL_ERR_NOT_SUPPORTED;
+  const SplitConfig c = default_split_config(products, (int)m, (int)n, (int)k, sm_count);
+  *tile_m = c.pair ? 256 : 128;
+  *tile_n = c.bn;
+  *split_k = c.splits;
+  return CORAL_OK;
+}
+
 coral_status_t coral_set_pair_raster(coral_handle_t hh, int group) {
   CORAL_HANDLE(hh);
   if (group < 0 || group > 64) return bad_arg(H, 1);

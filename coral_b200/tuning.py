@@ -99,18 +99,14 @@ def valid_mask(shapes: np.ndarray) -> np.ndarray:
 
 
 def default_choice(shape, sm_count: int = 148) -> int:
-    """Index in CANDIDATES of the library's default rule (no selector)."""
+    """Index in CANDIDATES of the library's default rule (no selector), as the library gives it."""
     m, n, k = (int(v) for v in shape[:3])
-    if -(-m // 256) * -(-n // 256) >= sm_count:
-        return CANDIDATES.index((256, 256, 1))
-    tn = 256 if shape_products(shape) == 3 else 128
-    tiles = -(-m // 128) * -(-n // 256)
-    sp = 1
-    if tiles * 2 <= sm_count and -(-k // 64) >= 16:
-        sp = min(16, max(1, sm_count // tiles))
-    sp = min(sp, max(1, -(-k // 64)))
-    best = max([s for s in (1, 2, 4, 8, 16) if s <= sp])
-    return CANDIDATES.index((128, tn, best))
+    tm, tn, sk = C.c_int(), C.c_int(), C.c_int()
+    st = _lib.load().coral_default_gemm_tile(shape_products(shape), m, n, k, sm_count, C.byref(tm), C.byref(tn),
+                                             C.byref(sk))
+    if st != 0:
+        raise RuntimeError(f"coral_default_gemm_tile: {st}")
+    return CANDIDATES.index((tm.value, tn.value, sk.value))
 
 
 # ------------------------------------------------------------ autotune DB --

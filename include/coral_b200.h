@@ -492,6 +492,10 @@ coral_status_t coral_set_gemm_tile(coral_handle_t h, int tile_m, int tile_n, int
 /* The tile a split-BF16 SGEMM of this shape would use now. */
 coral_status_t coral_get_gemm_tile(coral_handle_t h, int products, int op_a, int op_b, size_t m,
                                    size_t n, size_t k, int* tile_m, int* tile_n, int* split_k);
+/* The same by the default rule alone, for a device of sm_count SMs; needs no
+ * handle and no device. */
+coral_status_t coral_default_gemm_tile(int products, size_t m, size_t n, size_t k, int sm_count,
+                                       int* tile_m, int* tile_n, int* split_k);
 /* M-tiles per raster group of the CTA-pair tiles (1..64; 0 restores 8). */
 coral_status_t coral_set_pair_raster(coral_handle_t h, int group);
 /* The configuration a split-BF16 SGEMM of this shape would use now. */
