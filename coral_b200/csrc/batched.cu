@@ -19,17 +19,17 @@
 // 16-deep K slabs double-buffered through shared memory.  The bf16-input
 // variant reads bf16 operands and accumulates in fp32.
 //
-// Batched TRSV: one CTA per instance, blocked right-looking substitution over
-// 64-row diagonal blocks.  One warp runs the chain (take the previous block off
+// Batched TRSV: one CTA per instance (a warp up to 32 rows), blocked right-looking
+// substitution over 64-row diagonal blocks.  One warp runs the chain (take the previous block off
 // the next 64 rows, solve their diagonal block, divide by the diagonal as
 // strlsv.rs:66-140 does) while the other seven take that previous block off
 // all rows further down (coalesced column streaming, 48 loads in flight per
 // thread) and copy the next diagonal block and the block below it to shared
-// memory, so the chain never waits for memory.  What bounds it: the chain of
-// the largest instance (about 2.3 us per 64 rows), then HBM.  Sizes log-uniform
-// in [32, 1024], 1024 instances, 330 MB: 383 -> 106 us (3.1 TB/s); one instance
-// of 1024 rows: 387 -> 55 us.  Of that, starting the longest instances first
-// gave 40 us; asking for the next panel through L2 prefetches cost 10 us (more
+// memory, so the chain waits for memory at its start only.  What bounds it: the
+// chain of the largest instance (3.5 us per 64 rows alone on the GPU, twice that
+// beside a second CTA and 3 TB/s of others), then HBM.  Sizes log-uniform in
+// [32, 1024], 1024 instances, 330 MB: 372 -> 107 us (3.1 TB/s); one instance of 1024
+// rows: 261 -> 56 us.  Of that, starting the longest instances first gave 40 us; asking for the next panel through L2 prefetches cost 10 us (more
 // instructions than it saved) and is not done; two rows per thread took 136 us,
 // four the same as three.  Transposed operators read the same memory by rows,
 // backward solves walk it from its end.
@@ -226,6 +226,15 @@ constexpr int kBTLd = 68;                  // column pitch of the diagonal block
 constexpr int kBTLs = 65;                  // and of the block below it
 constexpr int kRows = 3;                   // rows per thread of the update
 constexpr int kBTMaxX = 1024;              // right-hand sides up to here stay in shared memory
+constexpr int kBTWindow = 1024;            // instances ordered together
+
+// The window a CTA draws from.
+struct TrsvWindow {
+  TrsvProblem cur;               // the system at `drawn`, for the CTA as a whole
+  unsigned short ord[kBTWindow];
+  int w, local, big, units, first;
+  int drawn, next;
+};
 
 struct TrsvSmem {
   float D[2][kBT][kBTLd];   // [column][row]
@@ -234,7 +243,9 @@ struct TrsvSmem {
   float part[4][kBT];
   float inv[kBT];
   float x[kBTMaxX];
+  TrsvWindow win;
 };
+extern __shared__ __align__(16) unsigned char trsv_smem[];
 
 // The system in solve order: always lower triangular, element (i, j) of op(A)
 // at a[i * rs + j * cs], right-hand side i at x[i * xs].  A backward solve
@@ -382,38 +393,72 @@ __device__ __forceinline__ void trsv_solve(TrsvSmem& sm, int b, bool fast, const
   __syncwarp();
 }
 
-// Instance for a CTA: within each window of kBTWindow instances, the CTAs take
-// them in decreasing order of size class (quarters of an octave, input order
-// inside a class), so the longest solves start first.  Every CTA finds its own
-// instance from the window's sizes: no plan pass, no memory beyond its own.
-constexpr int kBTWindow = 1024, kBTClasses = 128;
+// Order of the solves: within each window of kBTWindow instances by decreasing size
+// class (quarters of an octave), so the longest start first.  A CTA sorts a window
+// by itself -- no plan pass, no memory beyond its own -- and then draws positions of
+// it from the window's ticket; with more windows than one it goes on to the next
+// that has any left.  Systems of up to kBTSmall rows come last in a window, a warp
+// each and eight to a ticket: with a CTA and a ticket each they cost the 74 KB and
+// the barriers of a large one (us: 1000 systems of 8 rows 20.5 -> 5.6, 100000 of 4
+// 1640 -> 86, 20000 of 32 331 -> 67).
+constexpr int kBTClasses = 128, kBTSmall = 32, kBTSmallClasses = 20;
+constexpr int kBTWarps = kBTThreads / 32;
+constexpr unsigned kBTSpent = 1u << 31;   // a ticket's mark: the window has no position left
 __device__ __forceinline__ int trsv_class(int n) {
-  if (n <= 0) return 0;
-  const int lg = 31 - __clz(n);
-  return lg * 4 + (lg >= 2 ? (n >> (lg - 2)) & 3 : 0);
+  const int v = n - 1;
+  if (v <= 0) return 0;
+  const int lg = 31 - __clz(v);
+  return lg * 4 + (lg >= 2 ? (v >> (lg - 2)) & 3 : 0);
 }
-__device__ __forceinline__ int trsv_pick(const TrsvProblem* __restrict__ probs, int count, int pos) {
-  constexpr int kPer = kBTWindow / kBTThreads;
-  __shared__ int hist[kBTClasses], warp_sum[kBTThreads / 32];
-  __shared__ int cls, rank, pick;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int base = pos / kBTWindow * kBTWindow, local = pos - base;
-  if (t < kBTClasses) hist[t] = 0;
+// threadIdx.x read anew: what is derived from it here is not kept over the solves,
+// which leave no register for it (200 bytes of spills against 32).
+__device__ __forceinline__ int tid_now() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+// Fills ord with the window's instances (from its first) in order, input order inside
+// a class: every CTA that sorts a window has to find the same.  Returns how many have
+// more than kBTSmall rows.  Called and left by all threads together; the buffers of
+// the diagonal blocks are free then.
+__device__ __forceinline__ int trsv_order(const TrsvProblem* __restrict__ probs, int count, int base, TrsvSmem& sm) {
+  constexpr int kPer = kBTWindow / kBTThreads, kRuns = kBTWindow / 32;   // a run: 32 instances
+  static_assert(sizeof(int) * kRuns * kBTClasses <= sizeof(sm.D), "the table lies over the diagonal blocks");
+  int(*table)[kBTClasses] = reinterpret_cast<int(*)[kBTClasses]>(&sm.D[0][0][0]);   // of a run: class -> count, place
+  __shared__ int start[kBTClasses], big;
+  const int t = tid_now(), lane = t & 31, warp = t >> 5;
   int key[kPer];
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
-    const int i = base + t * kPer + q;
+    const int i = base + q * kBTThreads + t;
     key[q] = i < count ? trsv_class(probs[i].n) : -1;
   }
-  __syncthreads();
 #pragma unroll
-  for (int q = 0; q < kPer; ++q)
-    if (key[q] >= 0) atomicAdd(&hist[key[q]], 1);
+  for (int e = 0; e < kRuns * kBTClasses / kBTThreads; ++e) (&table[0][0])[e * kBTThreads + t] = 0;
   __syncthreads();
-  if (warp == 0) {  // classes from the top, 4 per lane
+  int rank[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const unsigned peers = __match_any_sync(0xffffffffu, key[q]);
+    rank[q] = __popc(peers & ((1u << lane) - 1u));
+    if (key[q] >= 0 && rank[q] == 0) table[q * kBTWarps + warp][key[q]] = __popc(peers);
+  }
+  __syncthreads();
+  if (t < kBTClasses) {
+    int run = 0;
+#pragma unroll 8
+    for (int r = 0; r < kRuns; ++r) {
+      const int c = table[r][t];
+      table[r][t] = run;
+      run += c;
+    }
+    start[t] = run;
+  }
+  __syncthreads();
+  if (warp == 0) {  // first position of each class: 4 classes a lane, from the top
     int h[4], sum = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) sum += h[q] = hist[kBTClasses - 1 - (lane * 4 + q)];
+    for (int q = 0; q < 4; ++q) sum += h[q] = start[kBTClasses - 1 - (lane * 4 + q)];
     int before = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -423,45 +468,24 @@ __device__ __forceinline__ int trsv_pick(const TrsvProblem* __restrict__ probs, 
     before -= sum;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      if (local >= before && local < before + h[q]) {
-        cls = kBTClasses - 1 - (lane * 4 + q);
-        rank = local - before;
-      }
+      const int c = kBTClasses - 1 - (lane * 4 + q);
+      start[c] = before;
       before += h[q];
+      if (c == kBTSmallClasses) big = before;
     }
   }
   __syncthreads();
-  int mine = 0;
-#pragma unroll
-  for (int q = 0; q < kPer; ++q) mine += key[q] == cls;
-  int before = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, before, o);
-    if (lane >= o) before += u;
-  }
-  if (lane == 31) warp_sum[warp] = before;
-  __syncthreads();
-  before -= mine;
-  for (int w = 0; w < warp; ++w) before += warp_sum[w];
 #pragma unroll
   for (int q = 0; q < kPer; ++q)
-    if (key[q] == cls && before++ == rank) pick = base + t * kPer + q;
+    if (key[q] >= 0)
+      sm.win.ord[start[key[q]] + table[q * kBTWarps + warp][key[q]] + rank[q]] = (unsigned short)(q * kBTThreads + t);
   __syncthreads();
-  return pick;
+  return big;
 }
 
-__global__ void __launch_bounds__(kBTThreads, 2)
-k_trsv_batched(const TrsvProblem* __restrict__ probs, int count, bool ordered) {
-  extern __shared__ __align__(16) unsigned char trsv_smem[];
-  TrsvSmem& sm = *reinterpret_cast<TrsvSmem*>(trsv_smem);
-  if ((int)blockIdx.x >= count) return;
-  const int pi = ordered ? trsv_pick(probs, count, blockIdx.x) : (int)blockIdx.x;
-  const TrsvProblem p = probs[pi];
-  if (p.n <= 0) return;
+// The system in solve order (see TrsvView).
+__device__ __forceinline__ TrsvView trsv_view(const TrsvProblem& p) {
   const bool t = p.trans != CORAL_NO_TRANSPOSE;
-  const bool lower_eff = (p.uplo == CORAL_LOWER) != t;
-  const bool unit = p.diag == CORAL_UNIT;
   TrsvView v;
   v.n = p.n;
   v.rs = t ? p.lda : 1;
@@ -469,13 +493,80 @@ k_trsv_batched(const TrsvProblem* __restrict__ probs, int count, bool ordered) {
   v.xs = p.incx;
   v.a = p.a;
   v.x = p.x;
-  if (!lower_eff) {
+  if ((p.uplo == CORAL_LOWER) == t) {
     v.a += (long long)(p.n - 1) * (1 + p.lda);
     v.x += (long long)(p.n - 1) * p.incx;
     v.rs = -v.rs;
     v.cs = -v.cs;
     v.xs = -v.xs;
   }
+  return v;
+}
+
+// One warp: a system of at most kBTSmall rows, lane = row, every load in flight.  As
+// in trsv_solve a product with the reciprocal and one correction stand for the
+// division, and divisions proper where they could round differently (a division per
+// row in the chain: 8 us for 32 rows).
+__device__ __noinline__ void trsv_small(const TrsvProblem& p) {
+  if (p.n <= 0) return;
+  const TrsvView v = trsv_view(p);
+  const int lane = threadIdx.x & 31, n = v.n;
+  const float* row = v.a + lane * v.rs;
+  const bool in = lane < n;
+  float a[kBTSmall];
+#pragma unroll
+  for (int g = 0; g < kBTSmall; g += 8)
+    if (g < n)
+#pragma unroll
+      for (int c = g; c < g + 8; ++c) a[c] = in && c < lane ? row[c * v.cs] : 0.f;
+  const float d = in && p.diag != CORAL_UNIT ? row[lane * v.cs] : 1.f;
+  const float rhs = in ? v.x[lane * v.xs] : 0.f;
+  const float inv = 1.f / d;
+  float r = rhs;
+#pragma unroll
+  for (int g = 0; g < kBTSmall; g += 8)
+    if (g < n)
+#pragma unroll
+      for (int c = g; c < g + 8; ++c) {
+        const float t = r * inv, x = fmaf(fmaf(-t, d, r), inv, t);
+        const float xc = __shfl_sync(0xffffffffu, x, c);
+        r = lane > c ? fmaf(-a[c], xc, r) : lane == c ? x : r;
+      }
+  if (!__all_sync(0xffffffffu, fabsf(d) > 0x1p-60f && fabsf(d) < 0x1p60f && fabsf(r) < INFINITY)) {
+    r = rhs;
+#pragma unroll 1
+    for (int c = 0; c < n; ++c) {
+      const float x = __shfl_sync(0xffffffffu, r, c) / __shfl_sync(0xffffffffu, d, c);
+      if (lane == c) r = x;
+      if (in && lane > c) r = fmaf(-row[c * v.cs], x, r);
+    }
+  }
+  if (in) v.x[lane * v.xs] = r;
+}
+
+// First CTA that starts in window w, of `grid` CTAs over nwin windows.
+__device__ __forceinline__ int trsv_first_cta(int w, int nwin, int grid) { return (w * grid + nwin - 1) / nwin; }
+// One thread: the next position of the window, or -1.  Every CTA draws one position too
+// many.  With one window the CTA that draws the last of those returns the ticket to
+// zero; with more, a window without positions is marked.
+__device__ __noinline__ void trsv_draw(TrsvWindow& win, const TrsvProblem* __restrict__ probs, unsigned* tickets,
+                                       int nwin, int own) {
+  const unsigned units = win.units;
+  const unsigned d = own < (int)units ? (unsigned)own : win.first + atomicAdd(&tickets[win.w], 1u);
+  if (d >= units) {
+    if (nwin > 1) atomicOr(&tickets[win.w], kBTSpent);
+    else if (d - units == gridDim.x - 1) tickets[0] = 0u;
+  }
+  win.drawn = d < units ? (int)d : -1;
+  if (d < (unsigned)win.big) win.cur = probs[win.w * kBTWindow + win.ord[d]];
+}
+
+// One CTA: a system of any size.
+__device__ __forceinline__ void trsv_solve_cta(const TrsvProblem& pr, TrsvSmem& sm) {
+  const TrsvProblem p = pr;
+  if (p.n <= 0) return;
+  const bool t = p.trans != CORAL_NO_TRANSPOSE, unit = p.diag == CORAL_UNIT;
+  const TrsvView v = trsv_view(p);
   const int n = v.n, nblk = (n + kBT - 1) / kBT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool in_smem = n <= kBTMaxX;
@@ -611,6 +702,93 @@ k_trsv_batched(const TrsvProblem* __restrict__ probs, int count, bool ordered) {
   }
 }
 
+// Without tickets a CTA takes the instance of its index.  With them (one per window,
+// then the number of CTAs that have finished; all zero before and after) the CTAs
+// stay and draw.  Against a CTA per position, each of which looked its instance up (3
+// us): batches of many small systems gain most, 300 of 900 to 1300 rows 206 -> 204,
+// and where the longest system decides the end costs 1 us, the last draw (1024 in
+// [32, 1024] 106.2 -> 107.7).  Drawing while the last block is solved hid that, but
+// registers made the solve 4% slower.
+__global__ void __launch_bounds__(kBTThreads, 2)
+k_trsv_batched(const TrsvProblem* __restrict__ probs, int count, unsigned* tickets) {
+  TrsvSmem& sm = *reinterpret_cast<TrsvSmem*>(trsv_smem);
+  TrsvWindow& win = sm.win;   // (no register holds it over a solve)
+  const int nwin = (int)(((unsigned)count + kBTWindow - 1) / kBTWindow);
+  if (!tickets) {
+    if (tid_now() == 0) win.cur = probs[blockIdx.x];
+  } else if (tid_now() == 0) {
+    win.w = (int)(blockIdx.x * (unsigned)nwin / gridDim.x);
+    win.units = 0;   // nothing sorted yet
+    win.first = -1;  // nothing drawn yet
+  }
+  __syncthreads();
+  for (;;) {
+    if (tickets) {
+      if (win.units == 0) {
+        const int b = trsv_order(probs, count, win.w * kBTWindow, sm);
+        if (tid_now() == 0) {
+          win.local = min(kBTWindow, count - win.w * kBTWindow);
+          win.big = b;
+          win.units = b + (win.local - b + kBTWarps - 1) / kBTWarps;
+          const int f = trsv_first_cta(win.w, nwin, gridDim.x);
+          // first positions: the second half backwards, so that the CTA that shares an SM
+          // with the longest system starts on the shortest of this wave
+          int own = win.units;
+          if (win.first < 0) {
+            const int c = trsv_first_cta(win.w + 1, nwin, gridDim.x) - f, h = c / 2;
+            own = (int)blockIdx.x - f;
+            if (own >= h) own = h + (c - 1 - own);
+          }
+          win.first = min(win.units, trsv_first_cta(win.w + 1, nwin, gridDim.x) - f);
+          trsv_draw(win, probs, tickets, nwin, own);
+        }
+        __syncthreads();
+      }
+      const int u = win.drawn;
+      if (u < 0) {
+        // on to the next window that has a position left, if any
+        if (nwin == 1) break;
+        __syncthreads();
+        if (tid_now() == 0) win.next = nwin;
+        __syncthreads();
+        for (int i = 1 + tid_now(); i < nwin; i += kBTThreads)
+          if (!(*(volatile unsigned*)&tickets[(win.w + i) % nwin] & kBTSpent)) {
+            atomicMin(&win.next, i);
+            break;
+          }
+        __syncthreads();
+        if (win.next == nwin) break;
+        __syncthreads();
+        if (tid_now() == 0) {
+          win.w = (win.w + win.next) % nwin;
+          win.units = 0;
+        }
+        __syncthreads();
+        continue;
+      }
+      if (u >= win.big) {
+        __syncthreads();   // `drawn` is read
+        if (tid_now() == 0) trsv_draw(win, probs, tickets, nwin, win.units);
+        const int pos = win.big + (u - win.big) * kBTWarps + (tid_now() >> 5);
+        if (pos < win.local) trsv_small(probs[win.w * kBTWindow + win.ord[pos]]);
+        __syncthreads();
+        continue;
+      }
+    }
+    trsv_solve_cta(win.cur, sm);
+    if (!tickets) return;
+    __syncthreads();
+    if (tid_now() == 0) trsv_draw(win, probs, tickets, nwin, win.units);
+    __syncthreads();   // before the buffers are written again
+  }
+  // with more windows than one, the last CTA to come here returns the tickets to zero
+  if (nwin > 1 && tid_now() == 0) {
+    __threadfence();
+    if (atomicAdd(&tickets[nwin], 1u) == gridDim.x - 1)
+      for (int i = 0; i <= nwin; ++i) tickets[i] = 0u;
+  }
+}
+
 }  // namespace
 }  // namespace coral
 
@@ -679,9 +857,14 @@ coral_status_t coral_strsv_batched(coral_handle_t hh, size_t count,
                                        (int)sizeof(TrsvSmem)));
     attr_devices |= bit;
   }
+  // Past two CTAs per SM the order of the solves matters: fixed CTAs that draw.
+  // (More windows than there are counters, 33 million systems: input order.)
+  const size_t slots = (size_t)H->sm_count * 2, nwin = (count + kBTWindow - 1) / kBTWindow;
+  const bool ordered = count > slots && nwin < kTrsvFlagBase;
+  if (ordered) own_state(H);
   timed_begin(H);
-  k_trsv_batched<<<(unsigned)count, kBTThreads, sizeof(TrsvSmem), H->stream>>>(
-      reinterpret_cast<const TrsvProblem*>(problems), (int)count, count > (size_t)H->sm_count * 2);
+  k_trsv_batched<<<(unsigned)(ordered ? slots : count), kBTThreads, sizeof(TrsvSmem), H->stream>>>(
+      reinterpret_cast<const TrsvProblem*>(problems), (int)count, ordered ? H->counters : nullptr);
   coral_status_t s = launch_status(H);
   timed_end(H);
   return s;
