@@ -634,6 +634,9 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
       for (int item = blockIdx.x; item < total_items && !abort_flag; item += gridDim.x) {
         int kb_lo, kb_hi;
         const Item t = item_at(item);
+        // A box of B past the last row is not loaded: what lies in its place reaches
+        // accumulator columns that are not stored (4096 x 1 x 4096: 63.5 -> 54.0 us).
+        const int cols = t.cols > kSplitBoxN && t.col0 + kSplitBoxN >= ws_cols ? kSplitBoxN : t.cols;
         slab_range(item, kb_lo, kb_hi);
         // K-serpentine: items of odd waves walk their slabs downwards, so a
         // wave starts on the slabs the previous wave read last, which are
@@ -650,12 +653,12 @@ k_gemm_split(const __grid_constant__ SplitMaps maps, int kdim, int m_tiles, int 
           }
           if (*(volatile int*)&abort_flag) break;
           uint8_t* st = smem + (size_t)s * kStageBytes;
-          tc::mbar_expect_tx(&full_bar[s], kPieces * (kATile + (uint32_t)t.cols * kBK * 2));
+          tc::mbar_expect_tx(&full_bar[s], kPieces * (kATile + (uint32_t)cols * kBK * 2));
           for (int p = 0; p < kPieces; ++p) {
             tc::tma_load_2d(st + p * kATile, &maps.a[p], &full_bar[s], kb * kBK, t.mt * kBM);
 #pragma unroll
             for (int c = 0; c < BN; c += kSplitBoxN)
-              if (c < t.cols)
+              if (c < cols)
                 tc::tma_load_2d(st + kPieces * kATile + p * kBTile + c / kSplitBoxN * kBBox, &maps.b[p],
                                 &full_bar[s], kb * kBK, t.col0 + c);
           }
