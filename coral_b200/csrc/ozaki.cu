@@ -172,20 +172,22 @@ __device__ __forceinline__ void slice_value(double a, int ex, int8_t (&out)[S]) 
   }
 }
 
-// Real: dst[p][row][l] for op(X) rows (K contiguous).  A CTA slices 32 rows x
-// 128 K values through shared memory, 16 loads in flight per thread; a thread
-// writes 16 K values of a row, 16 bytes per slice (rows of kp bytes, a multiple
-// of 16).  Bound: HBM (8 B read, 7 B written per element); 4096^2: 70 ->
-// 50 us against the fp64 loop with byte stores (64 with words).
-template <int S, bool kKMajorSrc>
+// Real: dst[p][row][l] for op(X) rows (K contiguous).  A CTA slices 32 rows x kDepth
+// K values through shared memory, all of a thread's kDepth / 8 loads in flight; a
+// thread writes kDepth / 8 K values of a row, as many bytes per slice (rows of kp
+// bytes, a multiple of 16).  Bound: HBM (8 B read, 7 B written per element); 4096^2:
+// 70 -> 50 us against the fp64 loop with byte stores (64 with words).  With 128 K
+// values a matrix of few CTAs waits for 16 values one after the other: 32 there (see
+// launch_slices).
+template <int S, bool kKMajorSrc, int kDepth>
 __global__ void __launch_bounds__(256)
 k_slice_real(const double* __restrict__ X, size_t ld, int R, int Kd, const int* __restrict__ e,
              int8_t* __restrict__ dst, size_t kp, size_t piece) {
-  // element (r, l) at r * kPitch + l + l / 16: no bank conflicts either way
-  constexpr int kRows = 32, kDepth = 128, kPitch = 137, kPer = kRows * kDepth / 256;
+  // element (r, l) at r * kPitch + l + l / kPer: no bank conflicts either way
+  constexpr int kRows = 32, kPer = kRows * kDepth / 256, kPitch = kDepth + 9, kWords = kPer / 4;
   __shared__ double tile[kRows * kPitch];
   const int r0 = blockIdx.y * kRows, l0 = blockIdx.x * kDepth;
-  const int g = threadIdx.x & 7, row = threadIdx.x >> 3, r_out = r0 + row, l_out = l0 + 16 * g;
+  const int g = threadIdx.x & 7, row = threadIdx.x >> 3, r_out = r0 + row, l_out = l0 + kPer * g;
   const int ex = r_out < R ? e[r_out] : 0;
   double v[kPer];
 #pragma unroll
@@ -197,17 +199,17 @@ k_slice_real(const double* __restrict__ X, size_t ld, int R, int Kd, const int* 
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
     const int i = threadIdx.x + 256 * q, l = kKMajorSrc ? i % kDepth : i / kRows;
-    tile[(kKMajorSrc ? i / kDepth : i % kRows) * kPitch + l + l / 16] = v[q];
+    tile[(kKMajorSrc ? i / kDepth : i % kRows) * kPitch + l + l / kPer] = v[q];
   }
   __syncthreads();
   if (r_out >= R || l_out >= (int)kp) return;
-  uint32_t w[S][4];
+  uint32_t w[S][kWords];
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
+  for (int a = 0; a < kWords; ++a) {
     uint32_t negs = 0u;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const SliceBits s = slice_bits(tile[row * kPitch + 17 * g + 4 * a + b], ex);
+      const SliceBits s = slice_bits(tile[row * kPitch + (kPer + 1) * g + 4 * a + b], ex);
 #pragma unroll
       for (int p = 0; p < S; ++p) w[p][a] = (b ? w[p][a] : 0u) | slice_digit(s, p) << (8 * b);
       if (s.neg) negs |= 0xffu << (8 * b);
@@ -220,8 +222,26 @@ k_slice_real(const double* __restrict__ X, size_t ld, int R, int Kd, const int* 
   }
   int8_t* o = dst + (size_t)r_out * kp + l_out;
 #pragma unroll
-  for (int p = 0; p < S; ++p)
-    *reinterpret_cast<uint4*>(o + p * piece) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  for (int p = 0; p < S; ++p) {
+    if constexpr (kWords == 4)
+      *reinterpret_cast<uint4*>(o + p * piece) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    else
+      *reinterpret_cast<uint32_t*>(o + p * piece) = w[p][0];
+  }
+}
+
+// 128 K values per CTA once there is a CTA of them for every SM.
+template <int S>
+coral_status_t launch_slices(Handle* h, const double* X, size_t ld, int R, int Kd, bool kmajor, const int* e,
+                             int8_t* dst, size_t kp, size_t piece) {
+  const unsigned rows = (unsigned)((R + 31) / 32);
+  const dim3 deep((unsigned)((kp + 127) / 128), rows), flat((unsigned)((kp + 31) / 32), rows);
+  const bool many = (size_t)deep.x * rows >= (size_t)h->sm_count;
+  if (many && kmajor) k_slice_real<S, true, 128><<<deep, 256, 0, h->stream>>>(X, ld, R, Kd, e, dst, kp, piece);
+  else if (many) k_slice_real<S, false, 128><<<deep, 256, 0, h->stream>>>(X, ld, R, Kd, e, dst, kp, piece);
+  else if (kmajor) k_slice_real<S, true, 32><<<flat, 256, 0, h->stream>>>(X, ld, R, Kd, e, dst, kp, piece);
+  else k_slice_real<S, false, 32><<<flat, 256, 0, h->stream>>>(X, ld, R, Kd, e, dst, kp, piece);
+  return launch_status(h);
 }
 
 // Complex, 4M layout (see k_split_cplx in gemm_split.cu): A rows [Re | Im];
@@ -390,11 +410,81 @@ __device__ __forceinline__ void oz_drain(uint32_t acc, double (&sum)[kCols]) {
   }
 }
 
-template <int S, int BN>
+// Eight accumulator columns from col0 (complex: four columns of C) of one row, for the
+// kernel of single tiles: what is read of C and of the column exponents, then, apart
+// from it, the results.  (The other kernels' epilogue through these is 8% slower at
+// 2048^3: laid out at once the compiler moves the loads of all groups.)
+struct OzGroup {
+  double c[8];
+  int e[8];
+};
+__device__ __forceinline__ void oz_load(const OzEpi& ep, int row, int col0, OzGroup& g) {
+  const bool read_c = !(ep.beta_re == 0.0 && ep.beta_im == 0.0);
+  if (!ep.complex_out) {
+    const double* crow = ep.C + row;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int col = col0 + j;
+      g.c[j] = (read_c && col < ep.n) ? crow[(size_t)col * ep.ldc] : 0.0;
+      g.e[j] = col < ep.n ? max(ep.eb[col], -4000) : 0;
+    }
+  } else {
+    const double2* crow = reinterpret_cast<const double2*>(ep.C) + row;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int col = col0 / 2 + j;
+      const double2 c = (read_c && col < ep.n) ? crow[(size_t)col * ep.ldc] : make_double2(0.0, 0.0);
+      g.c[2 * j] = c.x;
+      g.c[2 * j + 1] = c.y;
+      g.e[2 * j] = col < ep.n ? max(ep.eb[2 * col], -4000) : 0;
+      g.e[2 * j + 1] = col < ep.n ? max(ep.eb[2 * col + 1], -4000) : 0;
+    }
+  }
+}
+__device__ __forceinline__ void oz_store(const OzEpi& ep, int row, int col0, int ei, const OzGroup& g,
+                                         const double* sum) {
+  const bool beta0 = ep.beta_re == 0.0 && ep.beta_im == 0.0;
+  const bool beta1 = ep.beta_re == 1.0 && ep.beta_im == 0.0;
+  if (!ep.complex_out) {
+    double* crow = ep.C + row;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int col = col0 + j;
+      if (col >= ep.n) continue;
+      const double v = ep.alpha_re * ldexp(sum[j], ei + g.e[j]);
+      crow[(size_t)col * ep.ldc] = beta0 ? v : beta1 ? g.c[j] + v : ep.beta_re * g.c[j] + v;
+    }
+  } else {
+    double2* crow = reinterpret_cast<double2*>(ep.C) + row;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int col = col0 / 2 + j;
+      if (col >= ep.n) continue;
+      const double ar = ldexp(sum[2 * j], ei + g.e[2 * j]), ai = ldexp(sum[2 * j + 1], ei + g.e[2 * j + 1]);
+      double2 v = make_double2(ep.alpha_re * ar - ep.alpha_im * ai, ep.alpha_re * ai + ep.alpha_im * ar);
+      if (!beta0) {
+        const double2 cv = make_double2(g.c[2 * j], g.c[2 * j + 1]);
+        if (beta1) { v.x += cv.x; v.y += cv.y; }
+        else {
+          v.x += ep.beta_re * cv.x - ep.beta_im * cv.y;
+          v.y += ep.beta_re * cv.y + ep.beta_im * cv.x;
+        }
+      }
+      crow[(size_t)col * ep.ldc] = v;
+    }
+  }
+}
+
+// kOnce: one tile per CTA and one chunk of K (BN = 64 only).  The epilogue then goes from
+// TMEM to C eight columns at a time, in a loop; laid out over all columns of a thread,
+// the code runs once and what it costs is fetching it (DGEMM calls, us, with the small
+// slicing tiles: 16^3 24.4 -> 18.4, 128^3 29.1 -> 25.0, 512^3 38.9 -> 34.8).
+template <int S, int BN, bool kOnce>
 __global__ void __launch_bounds__(kOzThreads, 1)
 k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_tiles,
              int chunk_kb, OzEpi ep, unsigned* status, uint64_t limit_ns) {
   static_assert(S == 7, "the passes are laid out for seven slices");
+  static_assert(!kOnce || BN == 64, "one pass");
   using P = OzPlan<BN>;
   constexpr uint32_t kATile = P::kATile, kBTile = P::kBTile;
   constexpr int kSlots = P::kSlots;
@@ -558,6 +648,35 @@ k_gemm_ozaki(const __grid_constant__ OzMaps maps, int kdim, int m_tiles, int n_t
     const bool beta1 = ep.beta_re == 1.0 && ep.beta_im == 0.0;
     int gc = 0;
     bool stop = false;
+    if constexpr (kOnce) {
+      int mt, nt;
+      oz_tile_coords(blockIdx.x, m_tiles, n_tiles, mt, nt);
+      const int row = mt * kOzBM + quad * 32 + lane, col0 = nt * BN + half * kCols;
+      const bool in = row < ep.m;
+      const int ei = in ? max(ep.ea[row], -4000) : 0;
+      OzGroup g;
+      if (in) oz_load(ep, row, col0, g);   // on its way while the products run
+      if (!tc::mbar_wait_warp(&acc_full, 0, limit_ns)) {
+        atomicOr(status, kStatusTimeout);
+        stop = true;
+      }
+      tc::tc_fence_after();
+      stop = stop || tc::flag_warp(&abort_flag);
+      const uint32_t acc = tmem + half * kCols + lane_base;
+#pragma unroll 1
+      for (int c = 0; c < kCols && !stop; c += 8) {
+        double sum[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        oz_drain<5, 8, BN>(acc + 3 * BN + c, sum);
+        oz_drain<2, 4, BN>(acc + c, sum);
+        if (in) {
+          const OzGroup now = g;
+          if (c + 8 < kCols) oz_load(ep, row, col0 + c + 8, g);
+          oz_store(ep, row, col0 + c, ei, now, sum);
+        }
+        __syncwarp();
+      }
+      stop = true;
+    }
     for (int tile = blockIdx.x; tile < total_tiles && !stop; tile += gridDim.x) {
       int mt, nt;
       oz_tile_coords(tile, m_tiles, n_tiles, mt, nt);
@@ -669,20 +788,20 @@ int oz_chunk_slabs() {
   return (int)(kmax / kOzBK);
 }
 
-template <int S, int BN>
+template <int S, int BN, bool kOnce>
 coral_status_t launch_ozaki(Handle* h, const OzMaps& maps, int mr, int nr, int kd, const OzEpi& ep) {
   const size_t smem = 2 * ((size_t)OzPlan<BN>::kHigh + OzPlan<BN>::kLow) + 1024;
   static uint64_t attr_devices = 0;  // bit d: attribute set on device d
   const uint64_t bit = h->device < 64 ? (1ull << h->device) : 0;
   if (!(attr_devices & bit) || !bit) {
-    CORAL_CUDA(h, cudaFuncSetAttribute(k_gemm_ozaki<S, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CORAL_CUDA(h, cudaFuncSetAttribute(k_gemm_ozaki<S, BN, kOnce>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_devices |= bit;
   }
   const int m_tiles = (mr + kOzBM - 1) / kOzBM, n_tiles = (nr + BN - 1) / BN;
   const int tiles = m_tiles * n_tiles;
   const int grid = tiles < h->sm_count ? tiles : h->sm_count;
   timed_begin(h);
-  k_gemm_ozaki<S, BN><<<grid, kOzThreads, smem, h->stream>>>(maps, kd, m_tiles, n_tiles, oz_chunk_slabs<S>(), ep,
+  k_gemm_ozaki<S, BN, kOnce><<<grid, kOzThreads, smem, h->stream>>>(maps, kd, m_tiles, n_tiles, oz_chunk_slabs<S>(), ep,
                                                              &h->words->status, h->wait_limit * 32ull);
   coral_status_t s = launch_status(h);
   timed_end(h);
@@ -710,7 +829,10 @@ coral_status_t run_ozaki_gemm(Handle* h, const int8_t* ap, size_t a_piece, int m
         !encode_slices_map(&maps.b[i], bp, kd, nr, S, kp, b_piece, kOzBK, bn, 3 + i))
       return CORAL_ERR_NOT_SUPPORTED;
   }
-  return bn == 128 ? launch_ozaki<S, 128>(h, maps, mr, nr, kd, ep) : launch_ozaki<S, 64>(h, maps, mr, nr, kd, ep);
+  if (bn == 128) return launch_ozaki<S, 128, false>(h, maps, mr, nr, kd, ep);
+  const long long tiles = (long long)((mr + kOzBM - 1) / kOzBM) * ((nr + 63) / 64);
+  if (tiles <= h->sm_count && slabs <= oz_chunk_slabs<S>()) return launch_ozaki<S, 64, true>(h, maps, mr, nr, kd, ep);
+  return launch_ozaki<S, 64, false>(h, maps, mr, nr, kd, ep);
 }
 
 constexpr int kOzSlices = 7;
@@ -751,14 +873,8 @@ coral_status_t dgemm_ozaki_core(Handle* h, char* sc, int op_a, int op_b, size_t 
   coral_status_t s = launch_row_exponent(h, A, lda, (int)m, (int)k, a_km, ea);
   if (s != CORAL_OK) return s;
   if ((s = launch_row_exponent(h, B, ldb, (int)n, (int)k, b_km, eb)) != CORAL_OK) return s;
-  dim3 gsa((unsigned)((kp + 127) / 128), (unsigned)((m + 31) / 32));
-  dim3 gsb((unsigned)((kp + 127) / 128), (unsigned)((n + 31) / 32));
-  if (a_km) k_slice_real<S, true><<<gsa, 256, 0, h->stream>>>(A, lda, (int)m, (int)k, ea, ap, kp, a_piece);
-  else k_slice_real<S, false><<<gsa, 256, 0, h->stream>>>(A, lda, (int)m, (int)k, ea, ap, kp, a_piece);
-  if ((s = launch_status(h)) != CORAL_OK) return s;
-  if (b_km) k_slice_real<S, true><<<gsb, 256, 0, h->stream>>>(B, ldb, (int)n, (int)k, eb, bp, kp, b_piece);
-  else k_slice_real<S, false><<<gsb, 256, 0, h->stream>>>(B, ldb, (int)n, (int)k, eb, bp, kp, b_piece);
-  if ((s = launch_status(h)) != CORAL_OK) return s;
+  if ((s = launch_slices<S>(h, A, lda, (int)m, (int)k, a_km, ea, ap, kp, a_piece)) != CORAL_OK) return s;
+  if ((s = launch_slices<S>(h, B, ldb, (int)n, (int)k, b_km, eb, bp, kp, b_piece)) != CORAL_OK) return s;
   OzEpi ep{C, ldc, (int)m, (int)n, ea, eb, alpha, 0.0, beta, 0.0, 0};
   return run_ozaki_gemm<S>(h, ap, a_piece, (int)m, bp, b_piece, (int)n, (int)k, kp, ep);
 }
