@@ -41,11 +41,13 @@
 //               add alpha * partial into C.
 // Bound: issue slots (55% busy, a quarter of the stalls on instruction fetch)
 // and the latency of the slabs; 4096 instances with sizes log-uniform in
-// [16, 512] (1.34 GB, a floor of 208 us): fp32 810 -> 488 us, bf16 807 -> 436.
-// 2000 of 128^3: 197 -> 111 us.  Timed apart (the other side's work left out):
-// producers 350 us, epilogue 295, control alone 190.  A batch of four
-// instances of 2000-2300 is 10% slower than with the earlier 16-byte loads
-// (570 -> 631 us): such sizes belong to coral_sgemm.
+// [16, 512] (1.34 GB, a floor of 208 us): fp32 810 -> 493 us, bf16 807 -> 460.
+// 2000 of 128^3: fp32 197 -> 111 us, bf16 186 -> 98.  Timed apart (the other
+// side's work left out): producers 350 us, epilogue 295, control alone 190.
+// Few large instances whose operands both lie along K are what the 16-byte
+// loads of the earlier form did better: 16 of 1024^3 transposed fp32 221 -> 250
+// us, one 4096^3 in bf16 653 -> 725; their other orders gain (fp32 337 -> 224,
+// bf16 1351 -> 562).  Wide loads here cost the batch above a fifth or more.
 // Every wait is bounded: a wait that gives up sets the handle's status word
 // (reported by coral_sync) and the CTA winds down.
 #include "common.cuh"
@@ -397,7 +399,12 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
   };
   // Consumer side of the tile queue: the j-th tile of this CTA, which stays valid
   // until release_tile(j) (one arrival per consumer warp).  A whole warp calls it,
-  // all of its lanes with the same answer (see mbar_wait_warp), or one lane.
+  // all of its lanes with the same answer, or one lane.  It is the only place where
+  // the producers and the epilogue leave: their waits inside a tile may give up lane
+  // by lane, so the tile is finished all the same, its slots not waited for and
+  // nothing of it stored.  A vote at each of these waits too costs 1.5% (501 us and
+  // 463 against 493 and 460 on the batch above); with no vote, where single lanes
+  // may leave and the rest meet at a full-warp barrier, it was 480 and 448.
   auto next_tile = [&](int j, bool whole_warp) -> const TileInfo* {
     const int q = j % kQueue;
     bool go = tc::mbar_wait(&tq_full[q], (j / kQueue) & 1, limit_ns);
@@ -457,9 +464,8 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
     const bool is_a = group < 2;
     const uint32_t piece_bytes = is_a ? kAPieceBytes : kBPieceBytes;
     int it0 = 0;  // running number of the tile's first slab
-    bool stop = false;
     const TileInfo* tp;
-    for (int j = 0; !stop && (tp = next_tile(j, true)); ++j) {
+    for (int j = 0; (tp = next_tile(j, true)); ++j) {
       const TileInfo& ti = *tp;
       const coral_sgemm_problem_t& p = ti.p;
       // C is read in the epilogue, a column at a time: bring it into L2 now
@@ -488,16 +494,13 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
 #pragma unroll
             for (int u = 0; u < kInFlight; ++u)
               if (b0 + u < nb) o.load(b0 + u, left, tid, v[u]);
-            if (b0 == 0 && it >= S && !tc::mbar_wait_warp(&empty_bar[s], ((it / S) - 1) & 1, limit_ns)) {
+            // no way out from here: the lanes go on together, see next_tile
+            if (b0 == 0 && it >= S && !tc::mbar_wait_or(&empty_bar[s], ((it / S) - 1) & 1, limit_ns, &abort_flag))
               give_up();
-              stop = true;
-              break;
-            }
 #pragma unroll
             for (int u = 0; u < kInFlight; ++u)
               if (b0 + u < nb) store_block<TIn, NPC>(o.along_k, st + (b0 + u) * 2048, piece_bytes, v[u]);
           }
-          if (stop) break;
           tc::fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(&full_bar[s]);
@@ -568,9 +571,8 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
     const int quad = warp & 3, half = (warp - kEpiWarp0) >> 2;  // rows; every other group of 16 columns
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
     int gc = 0;
-    bool stop = false;
     const TileInfo* tp;
-    for (int j = 0; !stop && (tp = next_tile(j, true)); ++j) {
+    for (int j = 0; (tp = next_tile(j, true)); ++j) {
       const int m0 = tp->m0, n0 = tp->n0, nslabs = tp->nslabs, m = tp->p.m;
       const int row = m0 + quad * 32 + lane;
       const int ncols = min(tp->bn, tp->p.n - n0);
@@ -613,11 +615,8 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
         };
         // the first 16 columns of C on their way while the products finish
         load_c(q, ncols - 16 * half);
-        if (!tc::mbar_wait_warp(&acc_full[b], (gc >> 1) & 1, limit_ns)) {
-          give_up();
-          stop = true;
-          break;
-        }
+        const bool ok = tc::mbar_wait_or(&acc_full[b], (gc >> 1) & 1, limit_ns, &abort_flag);
+        if (!ok) give_up();
         tc::tc_fence_after();
         for (int col0 = 16 * half; col0 < ncols; col0 += 32) {
           uint32_t r[16];
@@ -631,7 +630,7 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
           }
           // the next group's C before this group's stores
           load_c(q + 32 * ldc, ncols - col0 - 32);
-          if (in) {
+          if (in && ok) {
             float* to = q;
             if (ncols - col0 >= 16) {
 #pragma unroll

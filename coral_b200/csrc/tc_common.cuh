@@ -83,6 +83,17 @@ constexpr uint64_t kDrainNs = 1000000000ull;
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit_ns));
 }
+// mbar_wait() that a flag in shared memory ends too; lane by lane, so what follows
+// must not depend on the answer where the warp acts together.
+__device__ __forceinline__ bool mbar_wait_or(uint64_t* bar, uint32_t parity, uint64_t limit_ns, const int* flag) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const uint64_t t0 = globaltimer();
+  for (uint32_t i = 0; i < 0xffffffffu; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 63u) == 0 && (globaltimer() - t0 > limit_ns || *(const volatile int*)flag)) return false;
+  }
+  return false;
+}
 // Whether a flag in shared memory is set, with one answer for the warp.
 __device__ __forceinline__ bool flag_warp(const int* flag) {
   return __any_sync(0xffffffffu, *(const volatile int*)flag);
