@@ -20,17 +20,18 @@
 // variant reads bf16 operands and accumulates in fp32.
 //
 // Batched TRSV: one CTA per instance (a warp up to 32 rows), blocked right-looking
-// substitution over 64-row diagonal blocks.  One warp runs the chain (take the previous block off
-// the next 64 rows, solve their diagonal block, divide by the diagonal as
-// strlsv.rs:66-140 does) while the other seven take that previous block off
-// all rows further down (coalesced column streaming, 48 loads in flight per
+// substitution over 64-row diagonal blocks.  One warp runs the chain (take the
+// previous block off the next 64 rows, solve their diagonal block, divide by the
+// diagonal as strlsv.rs:66-140 does) while the other seven take that previous block
+// off all rows further down (coalesced column streaming, 48 loads in flight per
 // thread) and copy the next diagonal block and the block below it to shared
 // memory, so the chain waits for memory at its start only.  What bounds it: the
 // chain of the largest instance (3.5 us per 64 rows alone on the GPU, twice that
 // beside a second CTA and 3 TB/s of others), then HBM.  Sizes log-uniform in
 // [32, 1024], 1024 instances, 330 MB: 372 -> 107 us (3.1 TB/s); one instance of 1024
-// rows: 261 -> 56 us.  Of that, starting the longest instances first gave 40 us; asking for the next panel through L2 prefetches cost 10 us (more
-// instructions than it saved) and is not done; two rows per thread took 136 us,
+// rows: 261 -> 53 us.  Of that, starting the longest instances first gave 40 us;
+// asking for the next panel through L2 prefetches cost 10 us (more instructions
+// than it saved) and is not done; two rows per thread took 136 us,
 // four the same as three.  Transposed operators read the same memory by rows,
 // backward solves walk it from its end.
 #include "common.cuh"
@@ -705,9 +706,9 @@ __device__ __forceinline__ void trsv_solve_cta(const TrsvProblem& pr, TrsvSmem& 
 // Without tickets a CTA takes the instance of its index.  With them (one per window,
 // then the number of CTAs that have finished; all zero before and after) the CTAs
 // stay and draw.  Against a CTA per position, each of which looked its instance up (3
-// us): batches of many small systems gain most, 300 of 900 to 1300 rows 206 -> 204,
+// us): batches of many small systems gain most, 300 of 900 to 1300 rows 206 -> 201,
 // and where the longest system decides the end costs 1 us, the last draw (1024 in
-// [32, 1024] 106.2 -> 107.7).  Drawing while the last block is solved hid that, but
+// [32, 1024] 106.4 -> 107.2).  Drawing while the last block is solved hid that, but
 // registers made the solve 4% slower.
 __global__ void __launch_bounds__(kBTThreads, 2)
 k_trsv_batched(const TrsvProblem* __restrict__ probs, int count, unsigned* tickets) {

@@ -757,7 +757,8 @@ coral_status_t enqueue_gemm_native(Handle* h, int op_a, int op_b, size_t m, size
     k_scale_c<T><<<g, 256, 0, h->stream>>>((int)m, (int)n, beta, C, ldc);
     return launch_status(h);
   }
-  // the widest C that is accepted
+  // The widest C that is accepted.  The grid below would carry more; the limit stays so
+  // that a size is refused or not as it always was.
   constexpr size_t kMaxCols = 65535u * (std::is_same<T, float>::value ? 128u : sizeof(T) == 16 ? 32u : 64u);
   if (n > kMaxCols) return CORAL_ERR_NOT_SUPPORTED;
   // ConjugateTranspose on a real type means Transpose (sgemm.rs:97-103).
