@@ -707,9 +707,8 @@ __device__ __forceinline__ void trsv_solve_cta(const TrsvProblem& pr, TrsvSmem& 
 // then the number of CTAs that have finished; all zero before and after) the CTAs
 // stay and draw.  Against a CTA per position, each of which looked its instance up (3
 // us): batches of many small systems gain most, 300 of 900 to 1300 rows 206 -> 201,
-// and where the longest system decides the end costs 1 us, the last draw (1024 in
-// [32, 1024] 106.4 -> 107.2).  Drawing while the last block is solved hid that, but
-// registers made the solve 4% slower.
+// and where the longest system decides the end costs 1 us (1024 in [32, 1024] 106.4
+// -> 107.2).  Drawing while the last block is solved does not take that back.
 __global__ void __launch_bounds__(kBTThreads, 2)
 k_trsv_batched(const TrsvProblem* __restrict__ probs, int count, unsigned* tickets) {
   TrsvSmem& sm = *reinterpret_cast<TrsvSmem*>(trsv_smem);
