@@ -789,6 +789,24 @@ k_trsv_batched(const TrsvProblem* __restrict__ probs, int count, unsigned* ticke
   }
 }
 
+// The tickets of one call, zero before and after it; null: there are none to be had,
+// the solves go in input order.  Calls that may run at the same time have tickets of
+// their own.  The calls on streams take theirs in turn from a ring; a captured call
+// may run again beside any other, so it keeps its own (a word up to 1024 systems).
+unsigned* trsv_tickets(Handle* h, size_t nwin) {
+  const size_t need = nwin > 1 ? nwin + 1 : 1, ring = kTicketKept - kTrsvFlagBase;
+  if (capture_of(h->stream)) {
+    if (need > kCounterPool - kTicketKept - h->tickets_kept) return nullptr;
+    h->tickets_kept += need;
+    return h->counters + kTicketKept + h->tickets_kept - need;
+  }
+  if (need > ring) return nullptr;
+  own_state(h);   // the ring comes round
+  if (need > ring - h->ticket_next) h->ticket_next = 0;
+  h->ticket_next += need;
+  return h->counters + kTrsvFlagBase + h->ticket_next - need;
+}
+
 }  // namespace
 }  // namespace coral
 
@@ -858,13 +876,11 @@ coral_status_t coral_strsv_batched(coral_handle_t hh, size_t count,
     attr_devices |= bit;
   }
   // Past two CTAs per SM the order of the solves matters: fixed CTAs that draw.
-  // (More windows than there are counters, 33 million systems: input order.)
-  const size_t slots = (size_t)H->sm_count * 2, nwin = (count + kBTWindow - 1) / kBTWindow;
-  const bool ordered = count > slots && nwin < kTrsvFlagBase;
-  if (ordered) own_state(H);
+  const size_t slots = (size_t)H->sm_count * 2;
+  unsigned* tickets = count > slots ? trsv_tickets(H, (count + kBTWindow - 1) / kBTWindow) : nullptr;
   timed_begin(H);
-  k_trsv_batched<<<(unsigned)(ordered ? slots : count), kBTThreads, sizeof(TrsvSmem), H->stream>>>(
-      reinterpret_cast<const TrsvProblem*>(problems), (int)count, ordered ? H->counters : nullptr);
+  k_trsv_batched<<<(unsigned)(tickets ? slots : count), kBTThreads, sizeof(TrsvSmem), H->stream>>>(
+      reinterpret_cast<const TrsvProblem*>(problems), (int)count, tickets);
   coral_status_t s = launch_status(H);
   timed_end(H);
   return s;

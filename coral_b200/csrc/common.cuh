@@ -70,6 +70,7 @@ struct Handle {
   // Zeroed pool of per-tile arrival counters for single-launch multi-block
   // combines; every kernel returns the counters it used to zero.
   unsigned* counters = nullptr;
+  size_t ticket_next = 0, tickets_kept = 0;   // taken of the two areas of tickets
   // TRSV epoch-tagged solution slots ((epoch << 32) | float bits), zeroed when
   // (re)allocated so stale memory never carries a live epoch.
   unsigned long long* trsv_slots = nullptr;
@@ -85,10 +86,12 @@ struct Handle {
 void timed_begin(Handle* h);
 void timed_end(Handle* h);
 
-constexpr size_t kCounterPool = 1u << 16;
-// Counters [0, kTrsvFlagBase) are zero-reset arrival counters; the rest are
-// TRSV ready flags.
+constexpr size_t kCounterPool = 1u << 18;
+// Counters [0, kTrsvFlagBase) are zero-reset arrival counters, those up to
+// kTicketKept the tickets of batched TRSV calls, taken in turn, and the rest
+// those of captured ones, each of which keeps its own.
 constexpr size_t kTrsvFlagBase = 1u << 15;
+constexpr size_t kTicketKept = 1u << 16;
 
 // Fixed device-side bookkeeping; counters are returned to zero by the last
 // block of the reduction that used them, so the area stays reusable.
@@ -114,6 +117,8 @@ enum CounterSlot { kCtrDot = 0, kCtrNrm2 = 1, kCtrIamax = 2, kCtrGemv = 3, kCtrT
 // does it): if that state was last used on another stream, the handle's stream
 // waits for what is enqueued there.  Nothing to do on the same stream.
 void own_state(Handle* h);
+// The capture that a stream takes part in: 0 none, ~0 cannot be told.
+unsigned long long capture_of(cudaStream_t s);
 
 // Ensure the handle owns at least `bytes` of scratch; returns nullptr on failure.
 void* scratch(Handle* h, size_t bytes);

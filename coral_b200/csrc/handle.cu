@@ -21,7 +21,7 @@ coral_status_t cuda_status(Handle* h, cudaError_t err) {
 
 // The capture that `s` takes part in, 0 when it is not capturing, ~0 when that
 // cannot be told (the legacy stream beside a capture).
-static unsigned long long capture_of(cudaStream_t s) {
+unsigned long long capture_of(cudaStream_t s) {
   if (s == nullptr || s == cudaStreamLegacy) return 0;   // never captured
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
