@@ -41,7 +41,7 @@
 //               add alpha * partial into C.
 // Bound: issue slots (55% busy, a quarter of the stalls on instruction fetch)
 // and the latency of the slabs; 4096 instances with sizes log-uniform in
-// [16, 512] (1.34 GB, a floor of 208 us): fp32 810 -> 493 us, bf16 807 -> 460.
+// [16, 512] (1.34 GB, a floor of 208 us): fp32 810 -> 478 us, bf16 807 -> 450.
 // 2000 of 128^3: fp32 197 -> 111 us, bf16 186 -> 98.  Timed apart (the other
 // side's work left out): producers 350 us, epilogue 295, control alone 190.
 // Few large instances whose operands both lie along K are what the 16-byte
@@ -402,16 +402,18 @@ k_gemm_grouped_tc(const coral_sgemm_problem_t* __restrict__ probs, int count,
   // all of its lanes with the same answer, or one lane.  It is the only place where
   // the producers and the epilogue leave: their waits inside a tile may give up lane
   // by lane, so the tile is finished all the same, its slots not waited for and
-  // nothing of it stored.  A vote at each of these waits too costs 1.5% (501 us and
-  // 463 against 493 and 460 on the batch above); with no vote, where single lanes
-  // may leave and the rest meet at a full-warp barrier, it was 480 and 448.
+  // nothing of it stored.  On the batch above, fp32 and bf16: 478 us and 450, as with
+  // lanes that leave one by one and the rest at a full-warp barrier (480 and 448);
+  // with a vote here 494 and 460, with one at each wait too 501 and 463.
   auto next_tile = [&](int j, bool whole_warp) -> const TileInfo* {
     const int q = j % kQueue;
-    bool go = tc::mbar_wait(&tq_full[q], (j / kQueue) & 1, limit_ns);
-    if (!go) give_up();
-    go = go && !*(volatile int*)&abort_flag;
-    if (whole_warp) go = __all_sync(0xffffffffu, go);
-    return go && tq[q].more ? &tq[q] : nullptr;
+    if (!tc::mbar_wait(&tq_full[q], (j / kQueue) & 1, limit_ns)) give_up();
+    if (whole_warp) {
+      __syncwarp();   // a lane that gave up has set the flag, and lane 0 reads it for all
+      const int stop = *(volatile int*)&abort_flag;
+      return __shfl_sync(0xffffffffu, stop, 0) == 0 && tq[q].more ? &tq[q] : nullptr;
+    }
+    return !*(volatile int*)&abort_flag && tq[q].more ? &tq[q] : nullptr;
   };
   auto release_tile = [&](int j) { tc::mbar_arrive(&tq_empty[j % kQueue]); };
 
